@@ -26,6 +26,8 @@
 #include "engine.h"
 #include "hprqp_batch.h"
 #include "hprqp.h"
+#include "batch_device.cuh"
+#include "cluster_solve.h"
 #include "rowblock.cuh"
 
 #include <cuda_runtime.h>
@@ -36,7 +38,10 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <numeric>
+#include <queue>
 #include <thread>
 #include <vector>
 
@@ -75,98 +80,6 @@ constexpr size_t smem_limit(int bt) { return ctas_per_sm(bt) == 1 ? 200 * 1024 :
 // shared memory per SM up to which the gathered vectors use a pool (batch_launch)
 constexpr size_t kPoolPerSm = 64 * 1024, kReservedSmemPerCta = 1024;
 
-struct BInst {
-    long long q_nz, a_nz, at_nz;  // first entry of the instance's matrices
-    int q_rp, a_rp, at_rp;        // first row pointer
-    int var, row;                 // first variable / row in the packed vectors
-    int n, m;
-    int q_lg, a_lg, at_lg;        // log2 of the SpMV lane-group width of Q, A, A' (0..5)
-    double obj_constant;
-};
-
-struct BatchArgs {
-    int K;
-    const BInst *inst;
-    const int *order;
-    unsigned long long *counter;  // the work queue's two ends (take_instance)
-    const int *q_rp, *q_ci, *a_rp, *a_ci, *at_rp, *at_ci;
-    const double *q_v0, *a_v0, *at_v0, *c0, *l0, *u0, *AL0, *AU0;
-    double *q_v, *a_v, *at_v;  // scaled copies
-    double *ws;                // per-CTA workspace
-    size_t ws_stride;
-    int nmax, mmax;
-    int vec_smem;              // 1: the gathered vectors live in shared memory
-    // parameters
-    double stoptol;
-    long long max_iter;
-    double time_limit;
-    int check_iter;
-    int print_frequency;
-    int use_scaling;
-    unsigned long long t_start;  // globaltimer at launch (ns), set by CTA 0
-    // host-mapped flag set by hprqp_batch_request_abort (nonzero: stop);
-    // read by thread 0 of each CTA when an instance starts and every
-    // kAbortPoll iterations
-    const int *abort_flag;
-    // outputs (packed like the inputs)
-    double *x, *y, *z, *w;
-    int *status;
-    long long *iters;
-    double *pobj, *resid, *gap;
-    int *restarts;
-    unsigned long long *phase_clk;  // optional [grid x 8] clock64 totals per phase
-    unsigned char *active_x;  // 1 = variable at a bound (for the adjoint)
-    unsigned char *active_r;  // 1 = row at a bound
-    double *col_norm_out, *row_norm_out;  // scaling of each instance (for the adjoint)
-    // optional starting point in the caller's (unscaled) variables, packed
-    // like the outputs; nullptr = start from zero as the reference does
-    const double *x_start, *w_start, *y_start;
-    const double *sigma_start;  // per instance, optional (<= 0: from the data)
-    double *sigma_out;          // per instance: sigma at the end of the solve
-    double *seconds_out;        // per instance: device time from its start to its end on its CTA
-    // single-QP solves (solve_gpu of a small model runs as a batch of one):
-    // the time limit counts from the start of the instance's iteration loop,
-    // as the host loop's does (after setup); optional milestone, loop-time
-    // and log outputs
-    int time_from_loop;
-    long long *iter4_out, *iter6_out;  // first checked iteration with KKT < 1e-4 / 1e-6 (-1: none)
-    double *time4_out, *time6_out;     // loop seconds at those iterations
-    double *loop_seconds_out;          // loop seconds at the end
-    double *log_buf;                   // kLogFields doubles per printed iteration (instance 0 only)
-    int log_cap;
-    int *log_count;
-};
-
-// optional per-CTA phase clocks: 0 load+scale, 1 setup norms/diag, 2 power
-// iterations, 3 steps, 4 residuals, 5 m-norm, 6 sigma+restart, 7 total
-#define PHASE_T0() long long _pt0 = clock64()
-#define PHASE_ADD(k)                                                                       \
-    do {                                                                                   \
-        if (B.phase_clk && threadIdx.x == 0)                                               \
-            B.phase_clk[blockIdx.x * 8 + (k)] += (unsigned long long)(clock64() - _pt0);   \
-        _pt0 = clock64();                                                                  \
-    } while (0)
-
-__device__ __forceinline__ unsigned long long globaltimer_ns()
-{
-    unsigned long long t;
-    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-    return t;
-}
-
-constexpr int kAbortPoll = 16;  // iterations between reads of the host abort flag
-// one log record: iter, errRp, errRd, primal obj, dual obj, gap, sigma, loop seconds
-constexpr int kLogFields = 8;
-
-// the host's abort request (a system-scope read of host-mapped memory)
-__device__ __forceinline__ bool abort_requested(const int *flag)
-{
-    if (!flag) return false;
-    int v;
-    asm volatile("ld.relaxed.sys.global.s32 %0, [%1];" : "=r"(v) : "l"(flag) : "memory");
-    return v != 0;
-}
-
 // local CSR view of one instance's matrix
 struct LCsr {
     int nrow;
@@ -175,11 +88,6 @@ struct LCsr {
     const double *v;
     int lg;  // log2 of the lanes that share a row in cta_spmv
 };
-
-__device__ __forceinline__ double clampd(double v, double lo, double hi)
-{
-    return v < lo ? lo : (v > hi ? hi : v);
-}
 
 // fold per-thread values over the CTA; every thread gets the results
 template <int N, int kBW>
@@ -272,59 +180,6 @@ __device__ __forceinline__ void cta_spmv(const LCsr &M, const double *x, F &&f)
         }
         if (lane < nr) f(c0 + lane, mine);
     }
-}
-
-// CTA-shared control state of the instance being solved
-struct CtaState {
-    double sigma, lA, lQ;
-    int q_is_diag, noC;
-    int n, m;
-    // restart (HPRQPRestart, include/shared/types.h:177-193)
-    int restart_flag, first_restart;
-    double last_gap, current_gap, save_gap, weighted_norm, best_gap, best_sigma;
-    long long inner, times;
-    // residuals (HPRQPResiduals)
-    double rp, rd, kkt, pobj, dobj, gap;
-    double norm_b_org, norm_c_org, obj_constant;
-    int to_check, do_res, stop, final_status;
-    int aborted;  // the host asked the batch to stop (sticky for the instance)
-    int print_yes, got4, got6;
-    double red[16];
-    double scal[8];
-};
-
-struct Vecs {
-    double *c, *l, *u, *col_norm, *x, *x_bar, *x_hat, *w, *w_bar, *ATy, *ATy_bar, *ATdy, *Qw, *Qw_bar, *Qx,
-        *dQw, *QATdy, *dx, *dw, *z_bar, *tempv, *diag_Q, *fact1, *fact2, *fact, *fact_M, *last_x, *last_Qw,
-        *last_w, *last_ATy, *fac_c, *pn;
-    double *AL, *AU, *row_norm, *y, *y_bar, *Ax, *dy, *s, *last_y, *fac_r, *pz, *pq;
-};
-
-constexpr int kBatchNVecs = 32, kBatchMVecs = 12;
-
-static __device__ Vecs carve(double *base, int nmax, int mmax, double *smem_pool)
-{
-    Vecs V;
-    double **nv[kBatchNVecs] = {&V.c,      &V.l,      &V.u,      &V.col_norm, &V.x,     &V.x_bar,  &V.x_hat,
-                                &V.w,      &V.w_bar,  &V.ATy,    &V.ATy_bar,  &V.ATdy,  &V.Qw,     &V.Qw_bar,
-                                &V.Qx,     &V.dQw,    &V.QATdy,  &V.dx,       &V.dw,    &V.z_bar,  &V.tempv,
-                                &V.diag_Q, &V.fact1,  &V.fact2,  &V.fact,     &V.fact_M, &V.last_x, &V.last_Qw,
-                                &V.last_w, &V.last_ATy, &V.fac_c, &V.pn};
-    double **mv[kBatchMVecs] = {&V.AL, &V.AU, &V.row_norm, &V.y,     &V.y_bar, &V.Ax,
-                                &V.dy, &V.s,  &V.last_y,   &V.fac_r, &V.pz,    &V.pq};
-    const int na = (nmax + 31) & ~31, ma = (mmax + 31) & ~31;
-    for (int k = 0; k < kBatchNVecs; ++k) *nv[k] = base + (size_t)k * na;
-    for (int k = 0; k < kBatchMVecs; ++k) *mv[k] = base + (size_t)kBatchNVecs * na + (size_t)k * ma;
-    if (smem_pool) {
-        // the gather sources of the step, the residuals and the power iteration
-        V.w = smem_pool;
-        V.w_bar = smem_pool + na;
-        V.tempv = smem_pool + 2 * na;
-        V.x_bar = smem_pool + 3 * na;
-        V.y_bar = smem_pool + 4 * na;
-        V.y = smem_pool + 4 * na + ma;
-    }
-    return V;
 }
 
 template <int kBW>
@@ -438,36 +293,6 @@ static __device__ __forceinline__ int take_instance(unsigned long long *counter,
     return order[back ? K - 1 - (int)back_taken : (int)front_taken];
 }
 
-static __device__ __forceinline__ size_t adaptive_step_d(long long iter)
-{
-    long long step = 10;
-    if (iter == 0) return step;
-    while (iter / step >= 100) step *= 10;
-    return step;
-}
-
-// a % d == 0 for the iteration counters of thread 0, in 32-bit arithmetic
-// while both fit (every practical count; 64-bit division is a long software
-// sequence that the whole CTA would wait for at the next barrier)
-static __device__ __forceinline__ bool divides(long long a, long long d)
-{
-    if (a >= 0 && d > 0 && a <= 0x7fffffffLL && d <= 0x7fffffffLL) return (unsigned)a % (unsigned)d == 0u;
-    return a % d == 0;
-}
-
-// iter lies on the reference's adaptive print grid (src/shared/solver_backend.c
-// print steps: every 10 below 1000, every 100 below 10000, ...)
-static __device__ __forceinline__ bool on_print_grid(long long iter)
-{
-    if (iter >= 0 && iter <= 0x7fffffffLL) {
-        const unsigned it = (unsigned)iter;
-        unsigned step = 10;
-        while (it / step >= 100u && step <= 100000000u) step *= 10;
-        return it % step == 0u;
-    }
-    return iter % (long long)adaptive_step_d(iter) == 0;
-}
-
 template <int BT>
 __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const BatchArgs B)
 {
@@ -518,6 +343,7 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
                 B.restarts[k] = 0;
                 B.sigma_out[k] = 0.0;
                 B.seconds_out[k] = 0.0;
+                atomicAdd(B.finished, 1ull);
             }
             __syncthreads();
             continue;
@@ -704,6 +530,7 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
             S.inner = 0;
             S.times = 0;
             S.aborted = 0;
+            S.yield = 0;
         }
         __syncthreads();
 
@@ -1114,7 +941,10 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
         for (iter = 0;; ++iter) {
             if (tid == 0) {
                 const double el = 1e-9 * (double)(globaltimer_ns() - (B.time_from_loop ? loop_t0 : B.t_start));
-                if (iter % kAbortPoll == 0 && !S.aborted && abort_requested(B.abort_flag)) S.aborted = 1;
+                if (iter % kAbortPoll == 0) {
+                    if (!S.aborted && abort_requested(B.abort_flag)) S.aborted = 1;
+                    if (iter > 0) S.yield = yield_now(B, I);
+                }
                 // an abort request stops the instance like the time limit
                 const bool over = el > B.time_limit || S.aborted;
                 int print_yes = 0;
@@ -1131,6 +961,7 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
             }
             __syncthreads();
             PHASE_ADD(3);
+            if (S.yield) break;
             if (S.do_res) residuals(iter);
             PHASE_ADD(4);
             if (tid == 0) {
@@ -1208,6 +1039,32 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
             __syncthreads();
         }
 
+        if (S.yield) {
+            // hand the instance over; vectors in the shared-memory pool go to
+            // their places in the workspace
+            const Vecs H = carve(B.ws + (size_t)blockIdx.x * B.ws_stride, B.nmax, B.mmax, nullptr);
+            if (B.vec_smem) {
+                for (int i = tid; i < n; i += kBT) {
+                    H.w[i] = V.w[i];
+                    H.w_bar[i] = V.w_bar[i];
+                    H.x_bar[i] = V.x_bar[i];
+                }
+                for (int i = tid; i < m; i += kBT) {
+                    H.y[i] = V.y[i];
+                    H.y_bar[i] = V.y_bar[i];
+                }
+            }
+            if (tid == 0) {
+                BResume *r = B.resume_out + atomicAdd(B.resume_count, 1ull);
+                r->inst = k;
+                r->slot = B.slot0 + blockIdx.x;
+                r->iter = iter;
+                r->t0 = inst_t0;
+                r->S = S;
+            }
+            break;
+        }
+
         // ---- output (reference workspace.cu:427-511) ---------------------------
         for (int i = tid; i < n; i += kBT) {
             const double cn = V.col_norm[i];
@@ -1233,6 +1090,7 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
             B.sigma_out[k] = S.sigma;
             B.seconds_out[k] = 1e-9 * (double)(globaltimer_ns() - inst_t0);
             if (B.loop_seconds_out) B.loop_seconds_out[k] = 1e-9 * (double)(globaltimer_ns() - loop_t0);
+            atomicAdd(B.finished, 1ull);
         }
         __syncthreads();
     }
@@ -1470,16 +1328,37 @@ struct NoInitAlloc : std::allocator<T> {
 template <class T>
 using HostVec = std::vector<T, NoInitAlloc<T>>;
 
+namespace hpr {
+// one launch of a phase: `count` entries of the phase's work order from
+// `first`, solved by clusters of C CTAs (C = 0: by one CTA each, k_batch_solve)
+// in the arithmetic of a one-CTA shape of vw warps
+struct Group {
+    int vw, C;
+    size_t first, count;
+};
+constexpr int kMaxGroups = 12;                    // 2 shapes x {0, 1, 2, 4, 8, 16}
+constexpr int kCounters = kMaxGroups + 2;         // one queue per launch, finished, handed over
+constexpr int kFinished = kMaxGroups, kHandedOver = kMaxGroups + 1;
+}  // namespace hpr
+
 struct HPRQPBatch {
     int device = 0;
     int num_sms = 148;
     int cta_threads = 1024;  // threads per CTA of the solve and adjoint kernels (kBigCta or kSmallCta)
-    // kBigCta batches: the last k_mid instances of the solve's work order
-    // (mid_cta_instance) are solved by kMidCta CTAs in a launch of their own
-    // on `stream`, the others by kBigCta CTAs on stream_mid
-    size_t k_mid = 0;
-    cudaStream_t stream = nullptr, stream_mid = nullptr;
-    int ws_slots = 0, phase_slots = 0;  // per-CTA workspaces and phase counters allocated
+    // the launches of a solve's first phase: segments of its work order
+    std::vector<hpr::Group> groups;
+    cudaStream_t stream = nullptr;
+    std::vector<cudaStream_t> side;     // streams of a phase's second, third, ... launch
+    int ws_slots = 0, phase_slots = 0;  // workspaces and phase counters allocated
+    // instances handed from one phase to the next (allocated by the first
+    // solve with more than one phase): records of two phases, work order
+    // a part of a call that solves k_total instances counts the finished ones
+    // of all parts in one place
+    int k_total = 0;
+    unsigned long long *finished = nullptr;
+    std::vector<int> order, phase_ids;  // instances of the first and of the current phase's entries
+    hpr::BResume *resume[2] = {nullptr, nullptr};
+    int *resume_order = nullptr;
     size_t K = 0;
     std::vector<size_t> var_off, row_off;          // original packing (caller's layout)
     std::vector<int> n_k, m_k;                      // preprocessed sizes
@@ -1571,8 +1450,9 @@ static void batch_free(HPRQPBatch *b)
     for (auto &m : b->models) model_free(&m);
     b->models.clear();
     if (b->stream) cudaStreamDestroy(b->stream);
-    if (b->stream_mid) cudaStreamDestroy(b->stream_mid);
-    b->stream = b->stream_mid = nullptr;
+    for (auto &st : b->side) cudaStreamDestroy(st);
+    b->side.clear();
+    b->stream = nullptr;
 }
 
 // The per-instance SpMV autotuner: the lane-group width of cta_spmv for one
@@ -1681,6 +1561,259 @@ static bool mid_cta_instance(const HPRQPModel &M)
     using namespace hpr;
     return M.Q.ncol <= (size_t)kMidCta && M.A.nrow <= (size_t)kMidCta && instance_work(M) <= kMidCtaMaxWork;
 }
+
+}  // extern "C"
+
+namespace hpr {
+
+// dynamic shared memory of k_cluster_solve (one CTA per SM: all there is)
+static size_t cluster_smem_limit()
+{
+    return 227 * 1024 - 8 * 1024;  // 8 KB for its static shared memory
+}
+
+static void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int C, int grid, size_t smem,
+                           cudaStream_t stream)
+{
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kClThreads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+}
+
+static const void *cluster_kernel_of(int C, bool resident)
+{
+    switch (C) {
+    case 1: return cluster_kernel<1>(resident);
+    case 2: return cluster_kernel<2>(resident);
+    case 4: return cluster_kernel<4>(resident);
+    case 8: return cluster_kernel<8>(resident);
+    default: return cluster_kernel<16>(resident);
+    }
+}
+
+static cudaError_t cluster_launch_of(int C, bool resident, const cudaLaunchConfig_t &cfg, const ClusterArgs &P)
+{
+    switch (C) {
+    case 1: return cluster_launch<1>(resident, cfg, P);
+    case 2: return cluster_launch<2>(resident, cfg, P);
+    case 4: return cluster_launch<4>(resident, cfg, P);
+    case 8: return cluster_launch<8>(resident, cfg, P);
+    default: return cluster_launch<16>(resident, cfg, P);
+    }
+}
+
+// virtual warps of instance k: the warps of its one-CTA shape
+static int instance_vw(const HPRQPBatch *b, size_t k)
+{
+    return (b->cta_threads == kBigCta ? (mid_cta_instance(b->models[k]) ? kMidCta : kBigCta) : kSmallCta) / 32;
+}
+
+// bytes of shared memory the largest slice of a matrix takes when C CTAs
+// share its rows: every row in quads of its own (cluster_solve.cuh)
+static size_t cluster_slice_bytes(const HPRQPMatrixCSR &M, int vw, int C)
+{
+    const size_t rows = (size_t)(vw / C) * ((M.nrow + vw - 1) / vw);
+    size_t most = 0;
+    for (size_t r0 = 0; r0 < M.nrow; r0 += rows) {
+        size_t q = 0;
+        for (size_t r = r0; r < std::min(r0 + rows, M.nrow); ++r)
+            if (M.row_ptr[r + 1] > M.row_ptr[r]) q += ((M.row_ptr[r + 1] + 3) >> 2) - (M.row_ptr[r] >> 2);
+        most = std::max(most, q);
+    }
+    return 16 * (2 * most + ((most + 1) >> 1));
+}
+
+// whether instance k can be solved by a cluster of C CTAs: every CTA has
+// rows (the exchanges of a step order the CTAs through their rows) and the
+// vectors fit
+static bool cluster_fits(const HPRQPBatch *b, size_t k, int C)
+{
+    const long long n = (long long)b->models[k].Q.ncol, m = (long long)b->models[k].A.nrow;
+    const int vw = instance_vw(b, k);
+    if (vw % C != 0 || n < 1 || n > kClMaxLen || m > kClMaxLen) return false;
+    if (C > 1 && (m < 1 || (long long)(C - 1) * (vw / C) * ((n + vw - 1) / vw) >= n)) return false;
+    return cluster_vec_bytes((int)n, (int)m, vw, C) <= cluster_smem_limit();
+}
+
+static bool cluster_resident(const HPRQPBatch *b, size_t k, int C)
+{
+    const HPRQPModel &M = b->models[k];
+    const int vw = instance_vw(b, k);
+    return cluster_vec_bytes((int)M.Q.ncol, (int)M.A.nrow, vw, C) + cluster_slice_bytes(M.Q, vw, C) +
+               cluster_slice_bytes(M.A, vw, C) + cluster_slice_bytes(M.AT, vw, C) + 64 <=
+           cluster_smem_limit();
+}
+
+// clusters of C CTAs the device holds at once (asked once per device)
+static int max_clusters(int device, int sms, int C)
+{
+    if (C <= 1) return sms;
+    static std::mutex mu;
+    static std::map<std::pair<int, int>, int> known;
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known.find({device, C});
+    if (it != known.end()) return it->second;
+    const void *kern = cluster_kernel_of(C, true);
+    const size_t smem = cluster_smem_limit();
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    cluster_config(cfg, at, C, C, smem, nullptr);
+    int c = 0;
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+        (C > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
+        cudaOccupancyMaxActiveClusters(&c, kern, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        c = 0;
+    }
+    known[{device, C}] = c;
+    return c;
+}
+
+// Microseconds of one iteration of instance k, measured on the batch recipe
+// (all SMs busy, one iteration in ten with a residual check); E = entries an
+// iteration reads.  One CTA of k_batch_solve: n = 100 / 600 / 1000 / 2000
+// (E = 2 k / 20 k / 53 k / 218 k): 7.8 / 17.6 / 39 / 134.  Clusters: n = 600
+// C = 1 / 2 / 4: 21 / 10.2 / 7.5; n = 1000 C = 2 / 4 / 8 / 16: 25 / 10.5 /
+// 8.2 / 6.6; n = 2000 C = 4 / 8 / 16: 63 / 28 / 12.
+static double iteration_us(const HPRQPBatch *b, size_t k, int C)
+{
+    const HPRQPModel &M = b->models[k];
+    const double E = 2.0 * (double)(M.Q.nnz + M.A.nnz);
+    if (C == 0) return 7.0 + 0.6e-3 * E;
+    return 3.0 + 1.5e-3 * (double)M.Q.ncol + 0.8e-3 * E / C * (cluster_resident(b, k, C) ? 1.0 : 1.3) +
+           (C > 8 ? 0.25 : 0.0);
+}
+
+// Cluster sizes for instances that all run at once: everyone starts with one
+// CTA, then the instance with the longest iteration gets twice the SMs as
+// long as that shortens it and SMs are left.  `fresh`: k_batch_solve may
+// take an instance too (it cannot go on with a handed-over one).  Returns
+// false when an instance fits no kernel here.
+struct Item {
+    const HPRQPBatch *b;
+    size_t k;
+};
+
+static bool choose_clusters(const std::vector<Item> &items, bool fresh, std::vector<int> &C)
+{
+    const size_t N = items.size();
+    if (N == 0) return true;
+    const int device = items[0].b->device, sms = items[0].b->num_sms;
+    C.assign(N, 0);
+    std::vector<double> t(N);
+    std::priority_queue<std::pair<double, size_t>> longest;
+    int cap[5];
+    for (int l = 0; l < 5; ++l) cap[l] = max_clusters(device, sms, 1 << l);
+    for (size_t j = 0; j < N; ++j) {
+        const HPRQPBatch *b = items[j].b;
+        const size_t k = items[j].k;
+        int c = cluster_fits(b, k, 1) ? 1 : 0;
+        if (!c && !fresh) {  // smallest cluster that holds it
+            for (c = 2; c <= 16 && !cluster_fits(b, k, c); c <<= 1) {}
+            if (c > 16) return false;
+        }
+        t[j] = iteration_us(b, k, c);
+        if (fresh && c && iteration_us(b, k, 0) <= t[j]) {
+            c = 0;
+            t[j] = iteration_us(b, k, 0);
+        }
+        C[j] = c;
+        longest.push({t[j], j});
+    }
+    int used[5] = {0, 0, 0, 0, 0};  // clusters of each size (one CTA: size 1)
+    auto lg = [](int c) { return c >= 16 ? 4 : c >= 8 ? 3 : c >= 4 ? 2 : c >= 2 ? 1 : 0; };
+    for (size_t j = 0; j < N; ++j) ++used[lg(C[j])];
+    // a size's clusters, the larger ones counted by the share they take of it
+    auto fits = [&]() {
+        for (int l = 0; l < 5; ++l) {
+            int sum = 0;
+            for (int h = l; h < 5; ++h) sum += used[h] << (h - l);
+            if (sum > cap[l]) return false;
+        }
+        int ctas = 0;
+        for (int l = 0; l < 5; ++l) ctas += used[l] << l;
+        return ctas <= sms - (used[1] + used[2] + used[3] + used[4] > 0 ? sms / 16 : 0);
+    };
+    while (!longest.empty()) {
+        const size_t j = longest.top().second;
+        longest.pop();
+        const HPRQPBatch *b = items[j].b;
+        const size_t k = items[j].k;
+        int best = 0;
+        double tb = 0.97 * t[j];
+        for (int c = std::max(2, 2 * C[j]); c <= 16; c <<= 1)
+            if (cluster_fits(b, k, c)) {
+                const double tc = iteration_us(b, k, c);
+                if (tc < tb) best = c;
+                if (best) break;
+            }
+        if (!best) continue;
+        --used[lg(C[j])];
+        ++used[lg(best)];
+        if (!fits()) {
+            ++used[lg(C[j])];
+            --used[lg(best)];
+            break;
+        }
+        C[j] = best;
+        t[j] = iteration_us(b, k, best);
+        longest.push({t[j], j});
+    }
+    return true;
+}
+
+// entries grouped by one-CTA shape and cluster size into `order` and `groups`
+// (the smaller shape first; order[e] = entry e's index in ids)
+static void make_groups(const HPRQPBatch *b, const std::vector<int> &ids, const std::vector<int> &C,
+                        std::vector<int> &order, std::vector<Group> &groups)
+{
+    order.clear();
+    groups.clear();
+    for (int big = 0; big < 2; ++big)
+        for (int c : {16, 8, 4, 2, 1, 0}) {
+            Group g{0, c, order.size(), 0};
+            for (size_t j = 0; j < ids.size(); ++j) {
+                const int vw = instance_vw(b, (size_t)ids[j]);
+                if ((vw == kBigCta / 32) != (big == 1) || C[j] != c) continue;
+                g.vw = vw;
+                order.push_back((int)j);
+            }
+            g.count = order.size() - g.first;
+            if (g.count) groups.push_back(g);
+        }
+}
+
+// The first phase of a solve.  Batches of at most one instance per SM: all
+// run at once, SMs spread by choose_clusters.  Larger ones: one CTA per
+// instance, the kMidCta instances (mid_cta_instance) in a launch started
+// first, so that every small instance -- whose iteration counts vary most --
+// starts at once, and the others in a launch whose CTAs take the SMs as the
+// first one's finish.  On entry order holds all instances, largest first; on
+// return its first half is cut into b->groups.
+static HPRQPStatus first_phase(HPRQPBatch *b, std::vector<int> &order)
+{
+    const size_t K = b->K;
+    b->groups.clear();
+    std::vector<int> ids(order.begin(), order.begin() + K), C(K, 0), pos;
+    if (K <= (size_t)b->num_sms) {
+        std::vector<Item> items(K);
+        for (size_t e = 0; e < K; ++e) items[e] = {b, (size_t)ids[e]};
+        if (!choose_clusters(items, true, C)) return HPRQP_STATUS_NOT_IMPLEMENTED;
+    }
+    make_groups(b, ids, C, pos, b->groups);
+    for (size_t e = 0; e < K; ++e) order[e] = ids[pos[e]];
+    return HPRQP_STATUS_OK;
+}
+
+}  // namespace hpr
+
+extern "C" {
 
 static HPRQPStatus batch_create_impl(size_t K, const size_t *var_offsets, const size_t *row_offsets,
                                      const HPRQPMatrixCSR *Q, const HPRQPMatrixCSR *A, const double *c,
@@ -1826,6 +1959,8 @@ static HPRQPStatus batch_create_impl(size_t K, const size_t *var_offsets, const 
         I.n = (int)M.Q.ncol;
         I.m = (int)M.A.nrow;
         I.obj_constant = M.obj_constant;
+        I.movable = 0;
+        for (int C = 16; C >= 1; C >>= 1) I.movable |= cluster_fits(b, k, C);
         // every instance's entries start on a 4-entry (16-byte) boundary, so
         // cta_spmv can read aligned quads of indices and values
         qnz += (M.Q.nnz + 3) & ~size_t(3);
@@ -1917,8 +2052,7 @@ static HPRQPStatus batch_create_impl(size_t K, const size_t *var_offsets, const 
     };
     if (cudaSetDevice(device_number) != cudaSuccess ||
         cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, device_number) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&b->stream_mid, cudaStreamNonBlocking) != cudaSuccess)
+        cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
         return fail(HPRQP_STATUS_NOT_IMPLEMENTED);
     BatchArgs &G = b->args;
     G.K = (int)K;
@@ -1932,27 +2066,22 @@ static HPRQPStatus batch_create_impl(size_t K, const size_t *var_offsets, const 
     cv.add(&d_atci, h_atci.size()).add(&d_qv0, h_qv.size()).add(&d_av0, h_av.size()).add(&d_atv0, h_atv.size());
     cv.add(&G.q_v, h_qv.size()).add(&G.a_v, h_av.size()).add(&G.at_v, h_atv.size());
     cv.add(&d_c, h_c.size()).add(&d_l, h_l.size()).add(&d_u, h_u.size()).add(&d_AL, h_AL.size()).add(&d_AU, h_AU.size());
-    cv.add(&d_inst, K).add(&d_order, 2 * K).add(&d_counter, 2);
+    cv.add(&d_inst, K).add(&d_order, 2 * K).add(&d_counter, kCounters);
     cv.add(&G.x, h_c.size()).add(&G.z, h_c.size()).add(&G.w, h_c.size()).add(&G.y, h_AL.size());
     cv.add(&G.status, K).add(&G.iters, K).add(&G.pobj, K).add(&G.resid, K).add(&G.gap, K).add(&G.restarts, K);
     cv.add(&G.sigma_out, K).add(&G.seconds_out, K).add(&G.active_x, h_c.size()).add(&G.active_r, h_AL.size());
     cv.add(&G.col_norm_out, h_c.size()).add(&G.row_norm_out, h_AL.size()).add(&b->d_t0, 1);
     if ((st = cv.commit(b))) return fail(st);
     // work orders, largest instances first: the adjoint's (second half of
-    // d_order) over all instances; the solve's (first half) the same with,
-    // in a kBigCta batch, the k_mid instances for kMidCta CTAs moved to its
-    // end -- the kBigCta launch takes the first K - k_mid entries, the
-    // kMidCta launch the rest, each as a queue with two ends
+    // d_order) over all instances, the solve's (first half) cut into the
+    // first phase's launches
     std::vector<int> order(2 * K);
     std::iota(order.begin(), order.begin() + K, 0);
     std::stable_sort(order.begin(), order.begin() + K,
                      [&](int x, int y) { return instance_work(b->models[x]) > instance_work(b->models[y]); });
     std::copy(order.begin(), order.begin() + K, order.begin() + K);
-    b->k_mid = 0;
-    if (b->cta_threads == kBigCta) {
-        std::stable_partition(order.begin(), order.begin() + K, [&](int k) { return !mid_cta_instance(b->models[k]); });
-        for (size_t k = 0; k < K; ++k) b->k_mid += mid_cta_instance(b->models[k]);
-    }
+    if ((st = first_phase(b, order))) return fail(st);
+    b->order.assign(order.begin(), order.begin() + K);
     auto up = [&](void *d, const void *h, size_t bytes) {
         return cudaMemcpyAsync(d, h, bytes, cudaMemcpyHostToDevice, b->stream) == cudaSuccess;
     };
@@ -2014,14 +2143,15 @@ HPRQPStatus hprqp_batch_create(size_t K, const size_t *var_offsets, const size_t
 
 namespace hpr {
 
-// a launched solve (batch_launch) waiting for batch_finish: one launch, or
-// two (segments of the work order) timed from one start event
+// a launched phase of a solve, waiting for batch_finish: its launches, timed
+// from one start event
 struct SolveLaunch {
-    cudaEvent_t e0 = nullptr, e1[2] = {nullptr, nullptr};
+    cudaEvent_t e0 = nullptr, e1[kMaxGroups] = {};
+    std::vector<Group> groups;
+    int phase = 0, running = 0, yield_at = 0;
     unsigned long long *d_phase = nullptr;
-    int segments = 0;
-    int bt[2] = {0, 0}, grid[2] = {0, 0};
-    size_t smem[2] = {0, 0};
+    int grid[kMaxGroups] = {};
+    double ms = 0.0;  // of the phases that ended
 };
 
 static void solve_launch_release(SolveLaunch &L)
@@ -2029,44 +2159,51 @@ static void solve_launch_release(SolveLaunch &L)
     if (L.e0) cudaEventDestroy(L.e0);
     for (auto &e : L.e1)
         if (e) cudaEventDestroy(e);
-    L.e0 = L.e1[0] = L.e1[1] = nullptr;
+    L.e0 = nullptr;
+    for (auto &e : L.e1) e = nullptr;
 }
 
-// Start the solve of a batch and return; the launches' events and optional
-// phase clocks are in L.  A kBigCta batch with instances for kMidCta CTAs
-// (mid_cta_instance) runs them first, in a kMidCta launch on the batch's
-// stream, and the others in a kBigCta launch on stream_mid: the mid-size CTAs (one
-// per SM) start every small instance at once -- the ones whose iteration
-// counts vary most -- and the 1024-thread CTAs take the SMs as they finish.
-static HPRQPStatus batch_launch(HPRQPBatch *b, const HPRQPBatchParams *p, SolveLaunch &L)
+// Start the launches L.groups of a phase: `order` (device) and, after the
+// first phase, `in` (records) say what they solve; total: instances of the
+// phase over all parts of the call.
+static HPRQPStatus phase_launch(HPRQPBatch *b, SolveLaunch &L, const int *order, const BResume *in, int total)
 {
-    B_CK(cudaSetDevice(b->device));
     BatchArgs &G = b->args;
     const size_t na = ((size_t)G.nmax + 31) & ~size_t(31), ma = ((size_t)G.mmax + 31) & ~size_t(31);
     const size_t vec_bytes = (4 * na + 2 * ma) * sizeof(double);  // the gathered vectors
-    struct Seg {
-        size_t first, count;  // entries of the work order
-        int bt;
-        cudaStream_t stream;
-    };
-    Seg seg[2];
-    int ns = 0;
-    const size_t k_big = b->K - b->k_mid;
-    if (b->k_mid > 0) {
-        seg[ns] = {k_big, b->k_mid, kMidCta, b->stream};
-        ++ns;
-    }
-    if (k_big > 0) {
-        seg[ns] = {0, k_big, b->cta_threads, ns == 0 ? b->stream : b->stream_mid};
-        ++ns;
-    }
-    L.segments = ns;
+    const int ns = (int)L.groups.size();
     auto kern_of = [](int bt) {
         return bt == kBigCta ? k_batch_solve<kBigCta> : bt == kMidCta ? k_batch_solve<kMidCta> : k_batch_solve<kSmallCta>;
     };
-    int vec_smem[2] = {0, 0}, slots = 0, off[2] = {0, 0};
+    while ((int)b->side.size() + 1 < ns) {
+        cudaStream_t st = nullptr;
+        B_CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        b->side.push_back(st);
+    }
+    int vec_smem[kMaxGroups] = {}, slots = 0, off[kMaxGroups] = {}, ctas = 0, coff[kMaxGroups] = {};
+    bool res[kMaxGroups] = {};
+    size_t smem[kMaxGroups] = {};
+    L.running = 0;
     for (int s = 0; s < ns; ++s) {
-        const int bt = seg[s].bt;
+        const Group &g = L.groups[s];
+        const int bt = 32 * g.vw;
+        off[s] = slots;
+        coff[s] = ctas;
+        if (g.C > 0) {
+            res[s] = true;
+            for (size_t e = g.first; res[s] && e < g.first + g.count; ++e)
+                res[s] = cluster_resident(b, (size_t)b->phase_ids[e], g.C);
+            const void *kern = cluster_kernel_of(g.C, res[s]);
+            smem[s] = cluster_smem_limit();
+            B_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[s]));
+            if (g.C > 8) B_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+            const int clusters = std::max(1, std::min((int)g.count, max_clusters(b->device, b->num_sms, g.C)));
+            L.grid[s] = clusters * g.C;
+            slots += clusters;
+            ctas += L.grid[s];
+            L.running += clusters;
+            continue;
+        }
         auto kern = kern_of(bt);
         // The gathered vectors go to shared memory only while the carveout
         // that takes leaves most of the SM's 256 KB of unified L1 / shared
@@ -2082,18 +2219,19 @@ static HPRQPStatus batch_launch(HPRQPBatch *b, const HPRQPBatchParams *p, SolveL
         B_CK(cudaFuncGetAttributes(&fa, kern));
         const size_t pool_per_sm = (size_t)ctas_per_sm(bt) * (vec_bytes + fa.sharedSizeBytes + kReservedSmemPerCta);
         vec_smem[s] = HPR_BATCH_VEC_SMEM && vec_bytes <= smem_limit(bt) && pool_per_sm <= kPoolPerSm;
-        L.smem[s] = vec_smem[s] ? vec_bytes : 0;
-        B_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L.smem[s]));
+        smem[s] = vec_smem[s] ? vec_bytes : 0;
+        B_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[s]));
         int per_sm = 0;
-        B_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bt, L.smem[s]));
-        L.bt[s] = bt;
-        L.grid[s] = std::max(1, std::min((int)seg[s].count, b->num_sms * std::max(per_sm, 1)));
-        off[s] = slots;
+        B_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bt, smem[s]));
+        L.grid[s] = std::max(1, std::min((int)g.count, b->num_sms * std::max(per_sm, 1)));
         slots += L.grid[s];
+        ctas += L.grid[s];
+        L.running += L.grid[s];
     }
-    // per-CTA workspace of every launch (allocated lazily, kept for the next solves)
+    // per-CTA workspace of every launch (allocated lazily, kept for the next
+    // solves; a handed-over instance keeps its slot)
     const size_t stride = kBatchNVecs * na + kBatchMVecs * ma;
-    if (!G.ws || G.ws_stride != stride || b->ws_slots < slots) {
+    if (!in && (!G.ws || G.ws_stride != stride || b->ws_slots < slots)) {
         double *ws = nullptr;
         HPRQPStatus st = balloc(b, &ws, stride * (size_t)slots);
         if (st) return st;
@@ -2101,97 +2239,212 @@ static HPRQPStatus batch_launch(HPRQPBatch *b, const HPRQPBatchParams *p, SolveL
         G.ws_stride = stride;
         b->ws_slots = slots;
     }
+    const char *pe = getenv("HPRQP_B200_BATCH_PHASES");
+    unsigned long long *d_phase = nullptr;
+    if (pe && pe[0] == '1') {
+        if (!b->d_phase || b->phase_slots < ctas) {
+            HPRQPStatus st2 = balloc(b, &b->d_phase, (size_t)ctas * 8);
+            if (st2) return st2;
+            b->phase_slots = ctas;
+        }
+        d_phase = b->d_phase;
+        B_CK(cudaMemsetAsync(d_phase, 0, (size_t)ctas * 8 * sizeof(unsigned long long), b->stream));
+    }
+    L.d_phase = d_phase;
+    // the queues of this phase; the count of finished instances goes on
+    B_CK(cudaMemsetAsync(G.counter, 0, (in ? kMaxGroups : kCounters) * sizeof(*G.counter), b->stream));
+    if (in) B_CK(cudaMemsetAsync(G.counter + kHandedOver, 0, sizeof(*G.counter), b->stream));
+    // the next phase: with a quarter of the running instances left, each of
+    // them can have four times the SMs (400 QPs of the batch recipe, limit
+    // 20,000 iterations: 418 ms without, 296 ms with the phases 37, 9 and 2
+    // instances from the end; a phase costs about 0.1 ms)
+    const int running = std::min(std::max(L.running, std::min(total, b->num_sms)), b->num_sms);
+    L.yield_at = running >= 8 ? running / 4 : 0;
+    if (L.yield_at > 0 && !b->resume[0]) {
+        const size_t most = (size_t)std::max(slots, 2 * b->num_sms);
+        HPRQPStatus st;
+        if ((st = balloc(b, &b->resume[0], most)) || (st = balloc(b, &b->resume[1], most)) ||
+            (st = balloc(b, &b->resume_order, most)))
+            return st;
+    }
+    if (!L.e0) B_CK(cudaEventCreate(&L.e0));
+    for (int s = 0; s < ns; ++s)
+        if (!L.e1[s]) B_CK(cudaEventCreate(&L.e1[s]));
+    // the time limit counts from here (a single-QP solve times its own loop)
+    if (!in && !G.time_from_loop) {
+        k_batch_clock<<<1, 1, 0, b->stream>>>(b->d_t0);
+        count_launch();
+        unsigned long long h_t0 = 0;
+        B_CK(cudaMemcpyAsync(&h_t0, b->d_t0, sizeof(h_t0), cudaMemcpyDeviceToHost, b->stream));
+        B_CK(cudaStreamSynchronize(b->stream));
+        G.t_start = h_t0;
+    }
+    B_CK(cudaEventRecord(L.e0, b->stream));
+    cudaError_t err = cudaSuccess;
+    for (int s = 0; s < ns && err == cudaSuccess; ++s) {
+        const Group &g = L.groups[s];
+        BatchArgs A = G;
+        A.K = (int)g.count;
+        A.order = order + g.first;
+        A.counter = G.counter + s;
+        A.ws = G.ws + (size_t)off[s] * stride;
+        A.ws_all = G.ws;
+        A.slot0 = off[s];
+        A.vec_smem = vec_smem[s];
+        A.phase_clk = d_phase ? d_phase + (size_t)coff[s] * 8 : nullptr;
+        A.K_total = b->k_total ? b->k_total : (int)b->K;
+        A.yield_at = L.yield_at;
+        A.finished = b->finished ? b->finished : G.counter + kFinished;
+        A.resume_count = G.counter + kHandedOver;
+        A.resume_out = b->resume[L.phase & 1];
+        A.resume_in = in;
+        const cudaStream_t stream = s == 0 ? b->stream : b->side[s - 1];
+        if (s > 0) err = cudaStreamWaitEvent(stream, L.e0, 0);
+        if (err != cudaSuccess) break;
+        if (g.C > 0) {
+            ClusterArgs P;
+            P.B = A;
+            P.vw = g.vw;
+            P.smem_bytes = (int)smem[s];
+            cudaLaunchConfig_t cfg = {};
+            cudaLaunchAttribute at[1];
+            cluster_config(cfg, at, g.C, L.grid[s], smem[s], stream);
+            err = cluster_launch_of(g.C, res[s], cfg, P);
+        } else {
+            kern_of(32 * g.vw)<<<L.grid[s], 32 * g.vw, smem[s], stream>>>(A);
+        }
+        count_launch();
+        if (err == cudaSuccess) err = cudaGetLastError();
+        if (err == cudaSuccess) err = cudaEventRecord(L.e1[s], stream);
+    }
+    if (err != cudaSuccess) {
+        // nothing launched may still run when the caller frees the batch
+        cudaStreamSynchronize(b->stream);
+        for (auto &st : b->side) cudaStreamSynchronize(st);
+        B_CK(err);
+    }
+    return HPRQP_STATUS_OK;
+}
+
+// Start the solve of a batch and return.
+static HPRQPStatus batch_launch(HPRQPBatch *b, const HPRQPBatchParams *p, SolveLaunch &L)
+{
+    B_CK(cudaSetDevice(b->device));
+    BatchArgs &G = b->args;
     G.stoptol = p->stoptol;
     G.max_iter = (long long)std::min<size_t>(p->max_iter, (size_t)LLONG_MAX);
     G.time_limit = p->time_limit;
     G.check_iter = (int)p->check_iter;
     G.print_frequency = p->print_frequency;
     G.use_scaling = p->use_scaling;
-    unsigned long long *d_t0 = b->d_t0;
-    B_CK(cudaMemsetAsync(G.counter, 0, 2 * sizeof(*G.counter), b->stream));
-    k_batch_clock<<<1, 1, 0, b->stream>>>(d_t0);
-    count_launch();
-    unsigned long long h_t0 = 0;
-    B_CK(cudaMemcpyAsync(&h_t0, d_t0, sizeof(h_t0), cudaMemcpyDeviceToHost, b->stream));
-    B_CK(cudaStreamSynchronize(b->stream));
-    G.t_start = h_t0;
-    const char *pe = getenv("HPRQP_B200_BATCH_PHASES");
-    unsigned long long *d_phase = nullptr;
-    if (pe && pe[0] == '1') {
-        if (!b->d_phase || b->phase_slots < slots) {
-            HPRQPStatus st2 = balloc(b, &b->d_phase, (size_t)slots * 8);
-            if (st2) return st2;
-            b->phase_slots = slots;
-        }
-        d_phase = b->d_phase;
-        B_CK(cudaMemsetAsync(d_phase, 0, (size_t)slots * 8 * sizeof(unsigned long long), b->stream));
-    }
-    L.d_phase = d_phase;
-    B_CK(cudaEventCreate(&L.e0));
-    for (int s = 0; s < ns; ++s) B_CK(cudaEventCreate(&L.e1[s]));
-    B_CK(cudaEventRecord(L.e0, b->stream));
-    cudaError_t err = cudaSuccess;
-    for (int s = 0; s < ns && err == cudaSuccess; ++s) {
-        BatchArgs A = G;
-        A.K = (int)seg[s].count;
-        A.order = G.order + seg[s].first;
-        A.counter = G.counter + s;
-        A.ws = G.ws + (size_t)off[s] * stride;
-        A.vec_smem = vec_smem[s];
-        A.phase_clk = d_phase ? d_phase + (size_t)off[s] * 8 : nullptr;
-        if (seg[s].stream != b->stream) err = cudaStreamWaitEvent(seg[s].stream, L.e0, 0);
-        if (err != cudaSuccess) break;
-        kern_of(seg[s].bt)<<<L.grid[s], seg[s].bt, L.smem[s], seg[s].stream>>>(A);
-        count_launch();
-        err = cudaGetLastError();
-        if (err == cudaSuccess) err = cudaEventRecord(L.e1[s], seg[s].stream);
-    }
-    if (err != cudaSuccess) {
-        // nothing launched may still run when the caller frees the batch
-        cudaStreamSynchronize(b->stream);
-        cudaStreamSynchronize(b->stream_mid);
-        B_CK(err);
-    }
-    return HPRQP_STATUS_OK;
+    L.groups = b->groups;
+    L.phase = 0;
+    L.ms = 0.0;
+    b->phase_ids = b->order;
+    return phase_launch(b, L, G.order, nullptr, b->k_total ? b->k_total : (int)b->K);
 }
 
-// Wait for a launched solve, record its device time (start event to the end
-// of the last launch), print the optional phase clocks.
-static HPRQPStatus batch_finish(HPRQPBatch *b, SolveLaunch &L)
+// Wait for a phase's launches and add its device time (start event to the
+// end of the last launch); print the optional phase clocks.
+static HPRQPStatus phase_wait(HPRQPBatch *b, SolveLaunch &L)
 {
-    B_CK(cudaSetDevice(b->device));
     cudaError_t err = cudaSuccess;
     float ms = 0.f;
-    for (int s = 0; s < L.segments; ++s) {
+    for (size_t s = 0; s < L.groups.size(); ++s) {
         const cudaError_t e = cudaEventSynchronize(L.e1[s]);
         if (err == cudaSuccess) err = e;
         float t = 0.f;
         if (e == cudaSuccess && cudaEventElapsedTime(&t, L.e0, L.e1[s]) == cudaSuccess) ms = std::max(ms, t);
     }
-    solve_launch_release(L);
+    L.ms += ms;
     B_CK(err);
     B_CK(cudaGetLastError());
-    b->last_ms = ms;
-    b->solved = true;
-    // an abort request ends with the solve it stopped
-    if (b->h_abort) __atomic_store_n(b->h_abort, 0, __ATOMIC_SEQ_CST);
     if (L.d_phase) {
-        int slots = 0;
-        for (int s = 0; s < L.segments; ++s) slots += L.grid[s];
-        std::vector<unsigned long long> h((size_t)slots * 8);
+        int ctas = 0;
+        for (size_t s = 0; s < L.groups.size(); ++s) ctas += L.grid[s];
+        std::vector<unsigned long long> h((size_t)ctas * 8);
         B_CK(cudaMemcpy(h.data(), L.d_phase, h.size() * sizeof(unsigned long long), cudaMemcpyDeviceToHost));
         double tot[8] = {0};
-        for (int g = 0; g < slots; ++g)
+        for (int g = 0; g < ctas; ++g)
             for (int q = 0; q < 8; ++q) tot[q] += (double)h[(size_t)g * 8 + q];
         fprintf(stderr, "[hprqp-b200 batch phases, %% of CTA time] load+scale %.1f setup %.1f power %.1f steps %.1f "
                         "residuals %.1f m-norm %.1f sigma+restart %.1f (",
                 100 * tot[0] / tot[7], 100 * tot[1] / tot[7], 100 * tot[2] / tot[7], 100 * tot[3] / tot[7],
                 100 * tot[4] / tot[7], 100 * tot[5] / tot[7], 100 * tot[6] / tot[7]);
-        for (int s = 0; s < L.segments; ++s)
-            fprintf(stderr, "%s%d CTAs of %d threads, smem %zu", s ? "; " : "", L.grid[s], L.bt[s], L.smem[s]);
-        fprintf(stderr, ")\n");
+        for (size_t s = 0; s < L.groups.size(); ++s)
+            fprintf(stderr, "%s%zu QPs, %d CTAs for %d warps, clusters of %d", s ? "; " : "", L.groups[s].count,
+                    L.grid[s], L.groups[s].vw, L.groups[s].C);
+        fprintf(stderr, "), %.2f ms\n", ms);
     }
     return HPRQP_STATUS_OK;
+}
+
+// Wait for launched solves (of one batch, or of the parts of one call that
+// share the device): while their phases hand instances over, launch the next
+// ones on them.
+static HPRQPStatus batch_finish(HPRQPBatch *const *b, SolveLaunch *L, int parts)
+{
+    auto run = [&]() -> HPRQPStatus {
+        std::vector<char> live(parts, 1);
+        for (;;) {
+            std::vector<std::vector<BResume>> rec(parts);
+            std::vector<Item> items;
+            for (int p = 0; p < parts; ++p) {
+                if (!live[p]) continue;
+                B_CK(cudaSetDevice(b[p]->device));
+                HPRQPStatus st = phase_wait(b[p], L[p]);
+                if (st) return st;
+                live[p] = 0;
+                if (L[p].yield_at == 0) continue;
+                unsigned long long count = 0;
+                B_CK(cudaMemcpyAsync(&count, b[p]->args.counter + kHandedOver, sizeof(count), cudaMemcpyDeviceToHost,
+                                     b[p]->stream));
+                B_CK(cudaStreamSynchronize(b[p]->stream));
+                if (count == 0) continue;
+                rec[p].resize(count);
+                B_CK(cudaMemcpyAsync(rec[p].data(), b[p]->resume[L[p].phase & 1], count * sizeof(BResume),
+                                     cudaMemcpyDeviceToHost, b[p]->stream));
+                B_CK(cudaStreamSynchronize(b[p]->stream));
+                for (auto &r : rec[p]) items.push_back({b[p], (size_t)r.inst});
+            }
+            if (items.empty()) return HPRQP_STATUS_OK;
+            std::vector<int> C;
+            if (!choose_clusters(items, false, C)) return HPRQP_STATUS_NOT_IMPLEMENTED;
+            size_t at = 0;
+            for (int p = 0; p < parts; ++p) {
+                const size_t count = rec[p].size();
+                if (count == 0) continue;
+                std::vector<int> ids(count), order;
+                for (size_t j = 0; j < count; ++j) ids[j] = rec[p][j].inst;
+                make_groups(b[p], ids, std::vector<int>(C.begin() + at, C.begin() + at + count), order, L[p].groups);
+                at += count;
+                b[p]->phase_ids.resize(count);
+                for (size_t e = 0; e < count; ++e) b[p]->phase_ids[e] = ids[order[e]];
+                B_CK(cudaMemcpyAsync(b[p]->resume_order, order.data(), count * sizeof(int), cudaMemcpyHostToDevice,
+                                     b[p]->stream));
+                B_CK(cudaStreamSynchronize(b[p]->stream));
+                const BResume *in = b[p]->resume[L[p].phase & 1];
+                ++L[p].phase;
+                HPRQPStatus st = phase_launch(b[p], L[p], b[p]->resume_order, in, (int)items.size());
+                live[p] = 1;
+                if (st) return st;
+            }
+        }
+    };
+    HPRQPStatus st = run();
+    for (int p = 0; p < parts; ++p) {
+        if (st) {  // nothing launched may still run when the caller frees the batch
+            cudaStreamSynchronize(b[p]->stream);
+            for (auto &s : b[p]->side) cudaStreamSynchronize(s);
+        }
+        solve_launch_release(L[p]);
+        if (st) continue;
+        b[p]->last_ms = L[p].ms;
+        b[p]->solved = true;
+        // an abort request ends with the solve it stopped
+        if (b[p]->h_abort) __atomic_store_n(b[p]->h_abort, 0, __ATOMIC_SEQ_CST);
+    }
+    return st;
 }
 
 }  // namespace hpr
@@ -2208,7 +2461,7 @@ HPRQPStatus hprqp_batch_solve(HPRQPBatch *b, const HPRQPBatchParams *p)
         solve_launch_release(L);
         return st;
     }
-    return batch_finish(b, L);
+    return batch_finish(&b, &L, 1);
 }
 
 HPRQPStatus hprqp_batch_set_warm_start(HPRQPBatch *b, const double *x0, const double *y0, const double *w0,
@@ -2637,12 +2890,17 @@ static HPRQPStatus solve_batch_in_two(size_t K, const size_t *var_offsets, const
                                params->device_number, false, &b[part], false, 0, ids[part].size(), kBigCta,
                                ids[part].data());
         t_create[part] = now() - tc;
-        if (st == HPRQP_STATUS_OK) st = batch_launch(b[part], params, L[part]);
+        if (st == HPRQP_STATUS_OK) {
+            // instances are handed over when few of both parts are left
+            b[part]->k_total = (int)K;
+            b[part]->finished = b[0]->args.counter + kFinished;
+            st = batch_launch(b[part], params, L[part]);
+        }
         if (st == HPRQP_STATUS_OK) ++launched;
     }
     const double t1 = now();
-    for (int part = 0; part < launched; ++part) {
-        const HPRQPStatus s2 = batch_finish(b[part], L[part]);
+    if (launched) {
+        const HPRQPStatus s2 = batch_finish(b, L, launched);
         if (st == HPRQP_STATUS_OK) st = s2;
     }
     const double t2 = now();

@@ -1,0 +1,39 @@
+// Host side of k_cluster_solve (cluster_solve.cuh): its shape and launch.
+#pragma once
+
+#include "batch_device.cuh"
+
+#include <cuda_runtime.h>
+
+namespace hpr {
+
+constexpr int kClThreads = 256;
+constexpr int kClMaxLen = 8190;  // columns as 16-bit byte offsets, the zero entry included
+// doubles of shared memory per own row of an n- and an m-vector (odd: a warp's
+// rows fall on different banks)
+constexpr int kClNOwn = 11, kClMOwn = 5;
+
+struct ClusterArgs {
+    BatchArgs B;
+    int vw;          // virtual warps: warps of the one-CTA shape of these instances
+    int smem_bytes;  // dynamic shared memory of a CTA
+};
+
+// bytes of shared memory an instance's vectors take in a CTA of a cluster:
+// the gathered vectors, the own slices and the row pointers
+__host__ __device__ __forceinline__ size_t cluster_vec_bytes(int n, int m, int vw, int C)
+{
+    const size_t big = n > m ? n : m;
+    const size_t nl = (size_t)(vw / C) * ((n + vw - 1) / vw), ml = (size_t)(vw / C) * ((m + vw - 1) / vw);
+    const size_t d = ((n + 2) & ~1) + ((big + 2) & ~size_t(1)) + ((m + 2) & ~1) + kClNOwn * nl + kClMOwn * ml;
+    return 8 * (d + 1) + 4 * ((2 * (nl + 1) + ml + 1 + 3) & ~size_t(3));
+}
+
+// Kernel for clusters of C CTAs; resident: every instance's matrices fit the
+// CTAs' shared memory (no code for streaming them).
+template <int C>
+const void *cluster_kernel(bool resident);
+template <int C>
+cudaError_t cluster_launch(bool resident, const cudaLaunchConfig_t &cfg, const ClusterArgs &P);
+
+}  // namespace hpr
