@@ -74,6 +74,7 @@ struct Ctl {
 struct DState {
     int n = 0, m = 0;
     int q_is_diag = 0, noC = 0;
+    int q_only_diag = 0;  // Q stores exactly its n diagonal entries
     DCsr Q, A, AT;
     double *c, *l, *u, *AL, *AU, *row_norm, *col_norm;
     double *x, *x_bar, *x_hat, *w, *w_bar, *y, *y_bar, *Ax, *ATy, *ATy_bar, *ATdy, *Qw, *Qw_bar, *Qx,
@@ -121,18 +122,18 @@ struct EpiBase {
     {
         for (int k = 0; k < N; ++k) o[k] = kSum;
     }
-    __device__ void extra(Acc<N> &) const {}
+    __device__ void extra(Acc<N> &, int, int) const {}
 };
 
 // first kernel of a step: latch inner_next -> inner
-__device__ __forceinline__ void latch_inner(Ctl *c)
+__device__ __forceinline__ void latch_inner(Ctl *c, int cta)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) c->inner = c->inner_next;
+    if (cta == 0 && threadIdx.x == 0) c->inner = c->inner_next;
 }
 // last kernel of a step: inner_next = inner + 1
-__device__ __forceinline__ void bump_inner(Ctl *c)
+__device__ __forceinline__ void bump_inner(Ctl *c, int cta)
 {
-    if (blockIdx.x == 0 && threadIdx.x == 0) c->inner_next = c->inner + 1;
+    if (cta == 0 && threadIdx.x == 0) c->inner_next = c->inner + 1;
 }
 
 // ---- one HPR step, non-noC ------------------------------------------------
@@ -163,7 +164,7 @@ struct EpiZXW1 : EpiBase<0> {
         S.x[i] = k.h2 * xh + k.h1 * S.last_x[i];
         S.w_bar[i] = wb;
     }
-    __device__ void extra(Acc<0> &) const { latch_inner(S.ctl); }
+    __device__ void extra(Acc<0> &, int cta, int) const { latch_inner(S.ctl, cta); }
 };
 
 // K2: tempv = x_hat + sigma (Qw - Q w_bar).
@@ -176,10 +177,27 @@ struct EpiTempv : EpiBase<0> {
         const double sigma = S.ctl->sigma;
         S.tempv[i] = S.x_hat[i] + sigma * (S.Qw[i] - qwb);
     }
-    __device__ void extra(Acc<0> &) const
+    __device__ void extra(Acc<0> &, int cta, int) const
     {
-        if (bump) bump_inner(S.ctl);
+        if (bump) bump_inner(S.ctl, cta);
     }
+};
+
+// K1 and K2 of a Q that stores its diagonal and nothing else: row i of both
+// products needs entry i only, so one elementwise pass does them (portfolio
+// QP, n = 60,120: 17 us as two products, 5 us).
+template <bool FULL>
+struct EpiDiagStep : EpiBase<0> {
+    EpiZXW1<FULL> k1;
+    EpiTempv k2;
+    __device__ void row(int i, double, Acc<0> &a) const
+    {
+        const DState &S = k1.S;
+        const double q = S.Q.v[i];
+        k1.row(i, q * S.w[i], a);
+        k2.row(i, q * S.w_bar[i], a);
+    }
+    __device__ void extra(Acc<0> &, int cta, int) const { latch_inner(k1.S.ctl, cta); }
 };
 
 // K3: Ax = A tempv fused with the projection onto [AL, AU] and the Halpern
@@ -206,9 +224,9 @@ struct EpiY : EpiBase<0> {
         }
         S.y[i] = k.h2 * yh + k.h1 * S.last_y[i];
     }
-    __device__ void extra(Acc<0> &) const
+    __device__ void extra(Acc<0> &, int cta, int) const
     {
-        if (bump) bump_inner(S.ctl);
+        if (bump) bump_inner(S.ctl, cta);
     }
 };
 
@@ -234,7 +252,7 @@ struct EpiW2 : EpiBase<0> {
         S.w[i] = k.h1 * S.last_w[i] + k.h2 * (2.0 * wbn - wi);
         S.ATy[i] = k.h1 * S.last_ATy[i] + k.h2 * (2.0 * atyb - aty);
     }
-    __device__ void extra(Acc<0> &) const { bump_inner(S.ctl); }
+    __device__ void extra(Acc<0> &, int cta, int) const { bump_inner(S.ctl, cta); }
 };
 
 // ---- one HPR step, noC (>= 80% free variables) ----------------------------
@@ -267,7 +285,7 @@ struct EpiZXW1noC : EpiBase<0> {
         S.w_bar[i] = wb;
         S.w[i] = k.h2 * wh + k.h1 * S.last_w[i];
     }
-    __device__ void extra(Acc<0> &) const { latch_inner(S.ctl); }
+    __device__ void extra(Acc<0> &, int cta, int) const { latch_inner(S.ctl, cta); }
 };
 
 // K2n: Qw_bar = Q w_bar fused with the Halpern Qw update and tempv.
@@ -284,9 +302,9 @@ struct EpiQwNoC : EpiBase<0> {
         S.Qw[i] = k.h2 * (2.0 * qwb - qw) + k.h1 * S.last_Qw[i];
         S.tempv[i] = S.x_hat[i] + k.sigma * (qw - qwb);
     }
-    __device__ void extra(Acc<0> &) const
+    __device__ void extra(Acc<0> &, int cta, int) const
     {
-        if (bump) bump_inner(S.ctl);
+        if (bump) bump_inner(S.ctl, cta);
     }
 };
 
@@ -307,6 +325,8 @@ struct EpiStore : EpiBase<0> {
 __global__ void k_soc_project(const double *in, double *out, const double *lo, const double *up, int lin,
                               const int *off, int ncones)
 {
+    begin_dependents();
+    wait_prerequisites();
     const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
     for (int i = tid; i < lin; i += nth) out[i] = clampd(in[i], lo[i], up[i]);
     const int lane = threadIdx.x & 31, wid = tid >> 5, nw = nth >> 5;
@@ -359,7 +379,7 @@ struct EpiSocX1 : EpiBase<0> {
         S.Qw[i] = qw;
         S.tempv[i] = S.x[i] + sigma * (-qw + S.ATy[i] - S.c[i]);
     }
-    __device__ void extra(Acc<0> &) const { latch_inner(S.ctl); }
+    __device__ void extra(Acc<0> &, int cta, int) const { latch_inner(S.ctl, cta); }
 };
 
 // S3 (over n): x_bar = proj(tempv) is in place; z_bar, x_hat, Halpern x, w_bar
@@ -526,9 +546,9 @@ struct EpiMATdy : EpiBase<2> {
         S.ATdy[i] = v;
         a.v[0] += v * S.dx[i];
     }
-    __device__ void extra(Acc<2> &a) const
+    __device__ void extra(Acc<2> &a, int cta, int ctas) const
     {
-        for (int i = blockIdx.x * kThreads + threadIdx.x; i < S.m; i += gridDim.x * kThreads) {
+        for (int i = cta * kThreads + threadIdx.x; i < S.m; i += ctas * kThreads) {
             const double d = S.dy[i];
             a.v[1] += d * d;
         }
@@ -615,7 +635,7 @@ struct EpiRestart : EpiBase<0> {
             S.last_Qw[i] = q;
         }
     }
-    __device__ void extra(Acc<0> &) const
+    __device__ void extra(Acc<0> &, int cta, int) const
     {
         for (int i = blockIdx.x * kThreads + threadIdx.x; i < S.m; i += gridDim.x * kThreads) {
             const double yb = S.y_bar[i];
@@ -752,6 +772,8 @@ struct FinalizeArgs {
 
 __global__ void __launch_bounds__(kThreads) k_finalize(const FinalizeArgs args)
 {
+    begin_dependents();
+    wait_prerequisites();
     const FinalizeSet fs = args.set[blockIdx.x];
     __shared__ double s_w[kWarps];
     for (int k = 0; k < fs.nred; ++k) {
@@ -985,9 +1007,9 @@ struct Engine {
     std::vector<void *> allocs;
     double sigma = 1.0, lambda_A = 0.0, lambda_Q = 0.0;
     double obj_constant = 0.0, norm_b_org = 0.0, norm_c_org = 0.0;
-    // graphs of one step, partial / full
-    cudaGraphExec_t step_graph[2] = {nullptr, nullptr};
-    uint64_t step_launches[2] = {0, 0};
+    // graphs of one partial step, one full step, kRunSteps partial steps
+    cudaGraphExec_t step_graph[3] = {nullptr, nullptr, nullptr};
+    uint64_t step_launches[3] = {0, 0, 0};
     bool use_graphs = true;
 };
 
@@ -1020,7 +1042,11 @@ static HPRQPStatus upload_csr(Engine *e, const HPRQPMatrixCSR &h, DCsr &d)
     for (size_t r = 0; r <= h.nrow; ++r) rp[r] = (int)h.row_ptr[r];
     for (size_t k = 0; k < h.nnz; ++k) ci[k] = (int)h.col_ind[k];
     TilePlan plan;
-    build_tile_plan(rp, plan);
+    build_tile_plan(rp, plan, tile_cap(h.nnz, e->num_sms));
+    for (int4 &t : plan.tiles) {
+        t.z = rp[t.x];
+        t.w = rp[t.y];
+    }
     std::vector<unsigned char> heads;
     build_heads(rp, heads);
     HPRQPStatus st;
@@ -1028,7 +1054,7 @@ static HPRQPStatus upload_csr(Engine *e, const HPRQPMatrixCSR &h, DCsr &d)
     if ((st = dalloc(e, &d.rp, rp.size())) || (st = dalloc(e, &d.ci, npad)) || (st = dalloc(e, &d.v, npad)) ||
         (st = dalloc(e, &d.heads, heads.size())) || (st = dalloc(e, &d.tiles, nt ? nt : 1)) ||
         (st = dalloc(e, &d.chunks, nc ? nc : 1)) || (st = dalloc(e, &d.long_rows, nl ? nl : 1)) ||
-        (st = dalloc(e, &d.chunk_partial, nc ? nc : 1)) || (st = dalloc(e, &d.err, 1)))
+        (st = dalloc(e, &d.chunk_partial, nc ? nc : 1)) || (st = dalloc(e, &d.chunks_done, 1)))
         return st;
     d.staged = choose_staged(rp, ci);
     d.ntiles = (int)nt;
@@ -1037,7 +1063,7 @@ static HPRQPStatus upload_csr(Engine *e, const HPRQPMatrixCSR &h, DCsr &d)
     d.grid_main = std::max(1, (d.ntiles + kWarps - 1) / kWarps);
     d.grid_chunk = (d.nchunks + kWarps - 1) / kWarps;
     d.grid_long = d.nlong ? (d.nlong + kThreads - 1) / kThreads : 0;
-    HPR_CK(cudaMemsetAsync(d.err, 0, sizeof(int), e->stream));
+    HPR_CK(cudaMemsetAsync(d.chunks_done, 0, sizeof(unsigned), e->stream));
     HPR_CK(cudaMemcpyAsync(d.rp, rp.data(), rp.size() * sizeof(int), cudaMemcpyHostToDevice, e->stream));
     HPR_CK(cudaMemcpyAsync(d.ci, ci.data(), ci.size() * sizeof(int), cudaMemcpyHostToDevice, e->stream));
     HPR_CK(cudaMemsetAsync(d.v + h.nnz, 0, (npad - h.nnz) * sizeof(double), e->stream));  // zero padding
@@ -1062,22 +1088,32 @@ static int ew_grid(const Engine *e, int len)
     return std::max(1, std::min(g, e->num_sms * 4));
 }
 
+// a kernel that begins while the one before it ends (wait_prerequisites)
+template <class... P, class... A>
+static void launch_k(Engine *e, void (*kern)(P...), int grid, A... args)
+{
+    cudaLaunchConfig_t cfg = {};
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = e->stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, P(args)...);
+    count_launch();
+}
+
 template <class Epi>
 static void launch_rb_at(Engine *e, const DCsr &M, const double *x, Epi epi, size_t poff)
 {
     if (M.nrow == 0) return;
     epi.partials = e->partials + poff;
-    if (M.nchunks) {
-        k_chunks<<<M.grid_chunk, kThreads, 0, e->stream>>>(M, x);
-        count_launch();
-    }
-    if (M.staged) k_spmv_staged<Epi><<<M.grid_main, kThreads, 0, e->stream>>>(M, x, epi);
-    else k_spmv<Epi><<<M.grid_main, kThreads, 0, e->stream>>>(M, x, epi);
-    count_launch();
-    if (M.nlong) {
-        k_long_epi<Epi><<<M.grid_long, kThreads, 0, e->stream>>>(M, epi);
-        count_launch();
-    }
+    const int grid = M.grid_chunk + M.grid_main;
+    if (M.staged) launch_k(e, k_spmv_staged<Epi>, grid, M, x, epi);
+    else launch_k(e, k_spmv<Epi>, grid, M, x, epi);
+    if (M.grid_long > 1) launch_k(e, k_long_epi<Epi>, M.grid_long, M, epi);
 }
 
 template <class Epi>
@@ -1092,8 +1128,7 @@ static int launch_ew(Engine *e, int len, Epi epi, int partial_offset = 0)
     if (len <= 0) return 0;
     const int g = ew_grid(e, len);
     if (Epi::NRED > 0) epi.partials = e->partials + partial_offset;
-    k_elementwise<Epi><<<g, kThreads, 0, e->stream>>>(len, epi);
-    count_launch();
+    launch_k(e, k_elementwise<Epi>, g, len, epi);
     return g;
 }
 
@@ -1121,8 +1156,7 @@ static HPRQPStatus finalize(Engine *e, const FinSpec *specs, int count, bool syn
         args.set[k].opsmask = specs[k].opsmask;
         args.set[k].out = e->dout->v + specs[k].out_off;
     }
-    k_finalize<<<count, kThreads, 0, e->stream>>>(args);
-    count_launch();
+    launch_k(e, k_finalize, count, args);
     if (sync) HPR_CK(cudaStreamSynchronize(e->stream));
     return HPRQP_STATUS_OK;
 }
@@ -1207,8 +1241,8 @@ static HPRQPStatus power_iteration(Engine *e, bool is_a, double *lambda_out)
 
 static void free_engine_memory(Engine *e)
 {
-    for (int k = 0; k < 2; ++k)
-        if (e->step_graph[k]) cudaGraphExecDestroy(e->step_graph[k]);
+    for (auto &g : e->step_graph)
+        if (g) cudaGraphExecDestroy(g);
     for (void *p : e->allocs) cudaFree(p);
     e->allocs.clear();
     if (e->hout) cudaFreeHost(e->hout);
@@ -1272,6 +1306,9 @@ HPRQPStatus engine_create(const HPRQPModel *model, const HPRQPParams *params, En
     S.n = n;
     S.m = m;
     E_ST(upload_csr(e, model->Q, S.Q));
+    S.q_only_diag = model->Q.nnz == model->Q.ncol;
+    for (int r = 0; S.q_only_diag && r < n; ++r)
+        S.q_only_diag = model->Q.row_ptr[r + 1] == (size_t)r + 1 && model->Q.col_ind[r] == (size_t)r;
     E_ST(upload_csr(e, model->A, S.A));
     E_ST(upload_csr(e, model->AT, S.AT));
     HPR_TRACE("create: csr uploaded");
@@ -1482,8 +1519,7 @@ static void enqueue_soc_step(Engine *e)
     EpiSocX1 k1;
     k1.S = S;
     launch_rb(e, S.Q, S.w, k1);
-    k_soc_project<<<pg, kThreads, 0, e->stream>>>(S.tempv, S.x_bar, S.l, S.u, S.lin_n, S.vco, S.nvc);
-    count_launch();
+    launch_k(e, k_soc_project, pg, (const double *)S.tempv, S.x_bar, S.l, S.u, S.lin_n, S.vco, S.nvc);
     EpiSocXFinish fx;
     fx.S = S;
     launch_ew(e, S.n, fx);
@@ -1494,8 +1530,7 @@ static void enqueue_soc_step(Engine *e)
         EpiSocY1 k3;
         k3.S = S;
         launch_rb(e, S.A, S.tempv, k3);
-        k_soc_project<<<pg, kThreads, 0, e->stream>>>(S.pz, S.s, S.AL, S.AU, S.lin_m, S.rco, S.nrc);
-        count_launch();
+        launch_k(e, k_soc_project, pg, S.pz, S.s, S.AL, S.AU, S.lin_m, S.rco, S.nrc);
         EpiSocYFinish fy;
         fy.S = S;
         launch_ew(e, S.m, fy);
@@ -1541,7 +1576,18 @@ static void enqueue_step(Engine *e, int to_check)
         }
         return;
     }
-    if (to_check) {
+    const bool diag_step = S.q_only_diag && S.m > 0;
+    if (diag_step) {
+        if (to_check) {
+            EpiDiagStep<true> k12;
+            k12.k1.S = k12.k2.S = S;
+            launch_ew(e, S.n, k12);
+        } else {
+            EpiDiagStep<false> k12;
+            k12.k1.S = k12.k2.S = S;
+            launch_ew(e, S.n, k12);
+        }
+    } else if (to_check) {
         EpiZXW1<true> k1;
         k1.S = S;
         launch_rb(e, S.Q, S.w, k1);
@@ -1551,9 +1597,11 @@ static void enqueue_step(Engine *e, int to_check)
         launch_rb(e, S.Q, S.w, k1);
     }
     if (S.m > 0) {
-        EpiTempv k2;
-        k2.S = S;
-        launch_rb(e, S.Q, S.w_bar, k2);
+        if (!diag_step) {
+            EpiTempv k2;
+            k2.S = S;
+            launch_rb(e, S.Q, S.w_bar, k2);
+        }
         if (to_check) {
             EpiY<true> k3;
             k3.S = S;
@@ -1576,33 +1624,51 @@ static void enqueue_step(Engine *e, int to_check)
 }
 
 
-static HPRQPStatus launch_step(Engine *e, int to_check)
+// Partial steps in one graph: the most that lie between two checks of the
+// first 1000 iterations (every 10; later runs are launched in pieces).  One
+// graph a step left the GPU idle between steps whenever a step's kernels are
+// shorter than the host's launch (n = 3001: 39 us a step, 37 with nine in a
+// graph, before the kernels themselves got shorter).
+constexpr int kRunSteps = 9;
+
+// one full step (kind 1), one partial step (0) or kRunSteps partial ones (2)
+static HPRQPStatus launch_step(Engine *e, int kind)
 {
-    to_check = to_check ? 1 : 0;
+    auto enqueue = [&]() {
+        for (int k = 0; k < (kind == 2 ? kRunSteps : 1); ++k) enqueue_step(e, kind == 1);
+    };
     if (!e->use_graphs) {
-        enqueue_step(e, to_check);
+        enqueue();
         return HPRQP_STATUS_OK;
     }
-    if (!e->step_graph[to_check]) {
+    if (!e->step_graph[kind]) {
         cudaGraph_t g;
         const uint64_t before = launch_count();
         HPR_CK(cudaStreamBeginCapture(e->stream, cudaStreamCaptureModeThreadLocal));
-        enqueue_step(e, to_check);
+        enqueue();
         HPR_CK(cudaStreamEndCapture(e->stream, &g));
-        e->step_launches[to_check] = launch_count() - before;
+        e->step_launches[kind] = launch_count() - before;
         g_launches.store(before);  // captured launches are counted at replay
-        HPR_CK(cudaGraphInstantiate(&e->step_graph[to_check], g, 0));
+        HPR_CK(cudaGraphInstantiate(&e->step_graph[kind], g, 0));
         cudaGraphDestroy(g);
     }
-    HPR_CK(cudaGraphLaunch(e->step_graph[to_check], e->stream));
-    count_launch(e->step_launches[to_check]);
+    HPR_CK(cudaGraphLaunch(e->step_graph[kind], e->stream));
+    count_launch(e->step_launches[kind]);
     return HPRQP_STATUS_OK;
 }
 
 HPRQPStatus engine_iteration_step(Engine *e, size_t inner, int to_check)
 {
     (void)inner;  // the Halpern counter is tracked on the device (Ctl)
-    return launch_step(e, to_check);
+    return launch_step(e, to_check ? 1 : 0);
+}
+
+HPRQPStatus engine_partial_steps(Engine *e, size_t count)
+{
+    HPRQPStatus st = HPRQP_STATUS_OK;
+    for (; st == HPRQP_STATUS_OK && count >= kRunSteps; count -= kRunSteps) st = launch_step(e, 2);
+    for (; st == HPRQP_STATUS_OK && count > 0; --count) st = launch_step(e, 0);
+    return st;
 }
 
 // ---- residuals ------------------------------------------------------------------
@@ -1636,16 +1702,14 @@ static HPRQPStatus engine_residuals_soc(Engine *e, HPRQPResiduals *res)
         ra.S = S;
         launch_rb_at(e, S.A, S.x_bar, ra, off_a);
         specs[ns++] = spec_of<EpiSocResA>(S.A.npart(), 0, off_a);
-        k_soc_project<<<pg, kThreads, 0, e->stream>>>(S.pq, S.pz, S.AL, S.AU, S.lin_m, S.rco, S.nrc);
-        count_launch();
+        launch_k(e, k_soc_project, pg, S.pq, S.pz, S.AL, S.AU, S.lin_m, S.rco, S.nrc);
         EpiSocRp rp;
         rp.S = S;
         const int g = launch_ew(e, S.m, rp, (int)off_rp);
         specs[ns++] = spec_of<EpiSocRp>(g, 16, off_rp);
     }
     const size_t off_v = off_rp + (size_t)e->num_sms * 4 * 3;
-    k_soc_project<<<pg, kThreads, 0, e->stream>>>(S.x_bar, S.ptmp, S.l, S.u, S.lin_n, S.vco, S.nvc);
-    count_launch();
+    launch_k(e, k_soc_project, pg, S.x_bar, S.ptmp, S.l, S.u, S.lin_n, S.vco, S.nvc);
     EpiSocViol vi;
     vi.S = S;
     const int gv = launch_ew(e, S.n, vi, (int)off_v);

@@ -31,6 +31,8 @@ void engine_destroy(Engine *e);
 // HPRQPSolverBackendOps (src/shared/solver_backend.h:18-36).
 HPRQPStatus engine_residuals(Engine *e, HPRQPResiduals *res, size_t iter);
 HPRQPStatus engine_iteration_step(Engine *e, size_t inner, int to_check);
+// count steps that no check follows, launched together
+HPRQPStatus engine_partial_steps(Engine *e, size_t count);
 HPRQPStatus engine_m_norm(Engine *e, double *out);
 HPRQPStatus engine_update_sigma(Engine *e, const HPRQPRestart *rst, const HPRQPResiduals *res,
                                 double *sigma_out);

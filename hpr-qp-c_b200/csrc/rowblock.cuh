@@ -63,23 +63,35 @@ struct DCsr {
     int *rp = nullptr;
     int *ci = nullptr;
     double *v = nullptr;    // ci and v hold padded_nnz(nnz) entries, the padding zero
-    int4 *tiles = nullptr;  // {r0, r1, entries, 0}
+    int4 *tiles = nullptr;  // {r0, r1, first entry, end}
     int ntiles = 0;
     int4 *chunks = nullptr;  // {row, k0, k1, slot}
     int nchunks = 0;
     int2 *long_rows = nullptr;  // {row, first chunk slot}
     int nlong = 0;
     double *chunk_partial = nullptr;
-    int *err = nullptr;
+    unsigned *chunks_done = nullptr;  // chunk CTAs that have stored their partials (0 between launches)
     unsigned char *heads = nullptr;  // bit j of heads[q]: entry 8q + j starts a non-empty row
     int staged = 0;      // 1: tiles run k_spmv_staged (rows of consecutive columns)
     int grid_main = 0;   // CTAs of k_spmv (one tile per warp)
-    int grid_chunk = 0;  // CTAs of k_chunks (8 chunks each)
-    int grid_long = 0;   // CTAs of k_long_epi
+    int grid_chunk = 0;  // CTAs for the chunks (8 each), the first ones of k_spmv's grid
+    int grid_long = 0;   // CTAs of k_long_epi; 1: the last chunk CTA does its work
     int npart() const { return grid_main + grid_long; }
 };
 
 enum RedOp : int { kSum = 0, kMax = 1 };
+
+// Programmatic dependent launch: the kernels of a step are short, and most of
+// a kernel's time is the chain of its first loads (tile, row starts, entries),
+// which do not depend on the kernel before it.  Every kernel that launch_k
+// starts reads what the setup fixed (plans, indices, matrix values), waits
+// for the kernels before it to end before it touches a vector, a scalar or a
+// partial, and lets the next one begin: a product when its sums are done (at
+// its start, the next kernel's CTAs take the places of a large product's
+// second wave: n = 200,000 138 us a step against 129), others at once.  The
+// step of an n = 3001 QP: 23.2 us without, 19.0 us with it.
+__device__ __forceinline__ void begin_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void wait_prerequisites() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 __device__ __forceinline__ double warp_sum(double v)
 {
@@ -138,8 +150,7 @@ __device__ __forceinline__ void block_reduce_store(Acc<N> &acc, const int *ops, 
 
 // sum of v[k] * x[ci[k]] over k = a + gl, a + gl + G, ... < e, four
 // independent loads in flight per step
-__device__ __forceinline__ double row_dot(const DCsr &M, const double *__restrict__ x, int a, int e, int gl,
-                                          int G)
+__device__ __forceinline__ double row_dot(const DCsr &M, const double *x, int a, int e, int gl, int G)
 {
     double s0 = 0.0, s1 = 0.0, s2 = 0.0, s3 = 0.0;
     int k = a + gl;
@@ -148,12 +159,12 @@ __device__ __forceinline__ double row_dot(const DCsr &M, const double *__restric
         const int c2 = __ldcs(M.ci + k + 2 * G), c3 = __ldcs(M.ci + k + 3 * G);
         const double v0 = __ldcs(M.v + k), v1 = __ldcs(M.v + k + G);
         const double v2 = __ldcs(M.v + k + 2 * G), v3 = __ldcs(M.v + k + 3 * G);
-        s0 = fma(v0, __ldg(x + c0), s0);
-        s1 = fma(v1, __ldg(x + c1), s1);
-        s2 = fma(v2, __ldg(x + c2), s2);
-        s3 = fma(v3, __ldg(x + c3), s3);
+        s0 = fma(v0, x[c0], s0);
+        s1 = fma(v1, x[c1], s1);
+        s2 = fma(v2, x[c2], s2);
+        s3 = fma(v3, x[c3], s3);
     }
-    for (; k < e; k += G) s0 = fma(__ldcs(M.v + k), __ldg(x + __ldcs(M.ci + k)), s0);
+    for (; k < e; k += G) s0 = fma(__ldcs(M.v + k), x[__ldcs(M.ci + k)], s0);
     return (s0 + s1) + (s2 + s3);
 }
 
@@ -168,8 +179,7 @@ __device__ __forceinline__ double row_dot(const DCsr &M, const double *__restric
 // order, writes the rows that start and end inside it, and hands the open
 // row across lanes with one segmented warp scan; the row still open at the
 // end of a window is carried into the next one.
-__device__ __forceinline__ void tile_rowsums(const DCsr &M, const double *__restrict__ x, int k0, int k1,
-                                             double *srow)
+__device__ __forceinline__ void tile_rowsums(const DCsr &M, const double *x, int k0, int k1, double *srow)
 {
     constexpr unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31;
@@ -204,6 +214,7 @@ __device__ __forceinline__ void tile_rowsums(const DCsr &M, const double *__rest
     };
     const int base0 = k0 & ~(kSpmvWinU - 1);
     if (base0 < k1) load(base0);
+    wait_prerequisites();
     for (int base = base0; base < k1; base += kSpmvWin) {
         const int e = base + kSpmvWinU * lane;
         int lo = k0 - e, hi = k1 - e;
@@ -212,7 +223,7 @@ __device__ __forceinline__ void tile_rowsums(const DCsr &M, const double *__rest
         const unsigned vm = hi > lo ? (((1u << hi) - 1u) & ~((1u << lo) - 1u)) : 0u;
         double p[kSpmvWinU];
 #pragma unroll
-        for (int j = 0; j < kSpmvWinU; ++j) p[j] = ((vm >> j) & 1u) ? v[j] * __ldg(x + c[j]) : 0.0;
+        for (int j = 0; j < kSpmvWinU; ++j) p[j] = ((vm >> j) & 1u) ? v[j] * x[c[j]] : 0.0;
         const unsigned h = hb & vm;
         load(base + kSpmvWin);  // the next window's stream, in flight while this one is summed
         int before = 0, total = 0;
@@ -260,20 +271,80 @@ __device__ __forceinline__ void tile_rowsums(const DCsr &M, const double *__rest
 // Epilogue concept:
 //   static constexpr int NRED;  __host__ __device__ void ops(int*) const;
 //   __device__ void init(Acc&) const; row(int i, double y_i, Acc&) const;
-//   __device__ void extra(Acc&) const;        // once per CTA, main kernel only
+//   __device__ void extra(Acc&, int cta, int ctas) const;  // once per CTA, tiles only
 //   double *partials;                         // [npart * NRED]
+// the long rows' epilogue: adds the chunk partials of row i in order
 template <class Epi>
-__global__ void __launch_bounds__(kThreads, HPR_SPMV_MIN_BLOCKS) k_spmv(const DCsr M, const double *__restrict__ xin, const Epi epi)
+__device__ __forceinline__ void long_rows(const DCsr &M, const Epi &epi, int cta)
+{
+    Acc<Epi::NRED> acc;
+    epi.init(acc);
+    const int i = cta * kThreads + threadIdx.x;
+    if (i < M.nlong) {
+        const int2 lr = M.long_rows[i];
+        const int c1 = i + 1 < M.nlong ? M.long_rows[i + 1].y : M.nchunks;
+        double s = 0.0;
+        for (int c = lr.y; c < c1; ++c) s += __ldcg(M.chunk_partial + c);
+        epi.row(lr.x, s, acc);
+    }
+    if constexpr (Epi::NRED > 0) {
+        int ops[Epi::NRED > 0 ? Epi::NRED : 1];
+        epi.ops(ops);
+        block_reduce_store<Epi::NRED>(acc, ops, epi.partials + (size_t)(M.grid_main + cta) * Epi::NRED);
+    }
+}
+
+// The chunk CTAs of a product (the first grid_chunk of its grid): one warp per
+// chunk of a long row.  The CTA that stores the last partial runs the long
+// rows' epilogue where one CTA holds them (grid_long = 1, up to 256 long
+// rows; with more, k_long_epi follows): one launch instead of three, and the
+// tiles run beside the chunks (portfolio QP, 120 rows of 60,000 entries and
+// 300 of 200: y = A x out of cold caches 44 us in three launches, 36 in one).
+template <class Epi>
+__device__ __forceinline__ void chunk_cta(const DCsr &M, const double *xin, const Epi &epi)
+{
+    __shared__ unsigned s_last;
+    const int lane = threadIdx.x & 31;
+    const int c = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    int4 C = make_int4(0, 0, 0, 0);
+    if (c < M.nchunks) C = M.chunks[c];
+    wait_prerequisites();
+    if (c < M.nchunks) {
+        double s = row_dot(M, xin, C.y, C.z, lane, 32);
+        s = warp_sum(s);
+        if (lane == 0) M.chunk_partial[C.w] = s;
+    }
+    begin_dependents();
+    if (M.grid_long != 1) return;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        s_last = atomicAdd(M.chunks_done, 1u) == (unsigned)M.grid_chunk - 1u;
+        if (s_last) *M.chunks_done = 0;
+        __threadfence();
+    }
+    __syncthreads();
+    if (s_last) long_rows(M, epi, 0);
+}
+
+template <class Epi>
+__global__ void __launch_bounds__(kThreads, HPR_SPMV_MIN_BLOCKS) k_spmv(const DCsr M, const double *xin, const Epi epi)
 {
     __shared__ double s_row[kWarps][kTileRows];
+    if ((int)blockIdx.x < M.grid_chunk) {
+        chunk_cta(M, xin, epi);
+        return;
+    }
+    const int cta = blockIdx.x - M.grid_chunk;
     Acc<Epi::NRED> acc;
     epi.init(acc);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int t = blockIdx.x * kWarps + wid;
+    const int t = cta * kWarps + wid;
     if (t < M.ntiles) {
         const int4 T = M.tiles[t];
         const int r0 = T.x, nr = T.y - T.x;
-        tile_rowsums(M, xin, __ldg(M.rp + r0), __ldg(M.rp + T.y), s_row[wid]);
+        tile_rowsums(M, xin, T.z, T.w, s_row[wid]);
+        begin_dependents();
         // ordinals of this lane's rows lane and lane + 32 among the tile's non-empty rows
         const unsigned lt = (1u << lane) - 1u;
         bool ne[2];
@@ -290,12 +361,14 @@ __global__ void __launch_bounds__(kThreads, HPR_SPMV_MIN_BLOCKS) k_spmv(const DC
             const int r = lane + 32 * j;
             if (r < nr) epi.row(r0 + r, ne[j] ? s_row[wid][ord[j]] : 0.0, acc);
         }
+    } else {
+        wait_prerequisites();
     }
-    epi.extra(acc);
+    epi.extra(acc, cta, M.grid_main);
     if constexpr (Epi::NRED > 0) {
         int ops[Epi::NRED > 0 ? Epi::NRED : 1];
         epi.ops(ops);
-        block_reduce_store<Epi::NRED>(acc, ops, epi.partials + (size_t)blockIdx.x * Epi::NRED);
+        block_reduce_store<Epi::NRED>(acc, ops, epi.partials + (size_t)cta * Epi::NRED);
     }
 }
 
@@ -309,7 +382,7 @@ __device__ __forceinline__ int win_slot(int i) { return i + (i >> 3); }
 // memory and a segmented scan there (head flags from the tile's row starts,
 // staged in shared memory) sums them per row into rowsum[0 .. nr - 1].
 // rs[0 .. nr] are the tile's row starts in shared memory.
-__device__ __forceinline__ void tile_rowsums_staged(const DCsr &M, const double *__restrict__ x, const int *rs, int nr,
+__device__ __forceinline__ void tile_rowsums_staged(const DCsr &M, const double *x, const int *rs, int nr,
                                              double *sv, unsigned char *sh, double *rowsum)
 {
     constexpr int KR = kTileRows / 32;
@@ -329,11 +402,12 @@ __device__ __forceinline__ void tile_rowsums_staged(const DCsr &M, const double 
         c[u] = k < k1 ? __ldcs(M.ci + k) : 0;
         v[u] = k < k1 ? __ldcs(M.v + k) : 0.0;
     }
+    wait_prerequisites();
     for (int base = k0; base < k1; base += kSpmvWin) {
         const int nb = base + kSpmvWin;
         double p[kSpmvWinU];
 #pragma unroll
-        for (int u = 0; u < kSpmvWinU; ++u) p[u] = v[u] * __ldg(x + c[u]);
+        for (int u = 0; u < kSpmvWinU; ++u) p[u] = v[u] * x[c[u]];
         // next window's stream, in flight while this one is summed
 #pragma unroll
         for (int u = 0; u < kSpmvWinU; ++u) {
@@ -411,16 +485,21 @@ __device__ __forceinline__ void tile_rowsums_staged(const DCsr &M, const double 
 }
 
 template <class Epi>
-__global__ void __launch_bounds__(kThreads, HPR_SPMV_STAGED_MIN_BLOCKS) k_spmv_staged(const DCsr M, const double *__restrict__ xin, const Epi epi)
+__global__ void __launch_bounds__(kThreads, HPR_SPMV_STAGED_MIN_BLOCKS) k_spmv_staged(const DCsr M, const double *xin, const Epi epi)
 {
     __shared__ double s_val[kWarps][kSpmvWin + kSpmvWin / 8];
     __shared__ unsigned char s_head[kWarps][kSpmvWin];
     __shared__ int s_rs[kWarps][kTileRows + 1];
     __shared__ double s_row[kWarps][kTileRows];
+    if ((int)blockIdx.x < M.grid_chunk) {
+        chunk_cta(M, xin, epi);
+        return;
+    }
+    const int cta = blockIdx.x - M.grid_chunk;
     Acc<Epi::NRED> acc;
     epi.init(acc);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int t = blockIdx.x * kWarps + wid;
+    const int t = cta * kWarps + wid;
     if (t < M.ntiles) {
         const int4 T = M.tiles[t];
         const int r0 = T.x, nr = T.y - T.x;
@@ -428,53 +507,31 @@ __global__ void __launch_bounds__(kThreads, HPR_SPMV_STAGED_MIN_BLOCKS) k_spmv_s
         for (int r = lane; r <= nr; r += 32) rs[r] = __ldg(M.rp + r0 + r);
         __syncwarp();
         tile_rowsums_staged(M, xin, rs, nr, s_val[wid], s_head[wid], s_row[wid]);
+        begin_dependents();
         __syncwarp();
 #pragma unroll
         for (int j = 0; j < kTileRows / 32; ++j) {
             const int r = lane + 32 * j;
             if (r < nr) epi.row(r0 + r, s_row[wid][r], acc);
         }
+    } else {
+        wait_prerequisites();
     }
-    epi.extra(acc);
+    epi.extra(acc, cta, M.grid_main);
     if constexpr (Epi::NRED > 0) {
         int ops[Epi::NRED > 0 ? Epi::NRED : 1];
         epi.ops(ops);
-        block_reduce_store<Epi::NRED>(acc, ops, epi.partials + (size_t)blockIdx.x * Epi::NRED);
+        block_reduce_store<Epi::NRED>(acc, ops, epi.partials + (size_t)cta * Epi::NRED);
     }
 }
 
-// one warp per chunk of a long row: partial sums only
-static __global__ void __launch_bounds__(kThreads) k_chunks(const DCsr M, const double *__restrict__ xin)
-{
-    const int lane = threadIdx.x & 31;
-    const int c = blockIdx.x * kWarps + (threadIdx.x >> 5);
-    if (c >= M.nchunks) return;
-    const int4 C = M.chunks[c];
-    double s = row_dot(M, xin, C.y, C.z, lane, 32);
-    s = warp_sum(s);
-    if (lane == 0) M.chunk_partial[C.w] = s;
-}
-
-// long rows: add the chunk partials in order and run the epilogue
+// the epilogue of more than 256 long rows, after k_spmv
 template <class Epi>
 __global__ void __launch_bounds__(kThreads) k_long_epi(const DCsr M, const Epi epi)
 {
-    Acc<Epi::NRED> acc;
-    epi.init(acc);
-    const int i = blockIdx.x * kThreads + threadIdx.x;
-    if (i < M.nlong) {
-        const int2 lr = M.long_rows[i];
-        const int c1 = i + 1 < M.nlong ? M.long_rows[i + 1].y : M.nchunks;
-        double s = 0.0;
-        for (int c = lr.y; c < c1; ++c) s += M.chunk_partial[c];
-        epi.row(lr.x, s, acc);
-    }
-    if constexpr (Epi::NRED > 0) {
-        int ops[Epi::NRED > 0 ? Epi::NRED : 1];
-        epi.ops(ops);
-        block_reduce_store<Epi::NRED>(acc, ops,
-                                      epi.partials + (size_t)(M.grid_main + blockIdx.x) * Epi::NRED);
-    }
+    begin_dependents();
+    wait_prerequisites();
+    long_rows(M, epi, blockIdx.x);
 }
 
 // Elementwise kernel over max(n, m) with the same epilogue/reduction
@@ -482,10 +539,12 @@ __global__ void __launch_bounds__(kThreads) k_long_epi(const DCsr M, const Epi e
 template <class Epi>
 __global__ void __launch_bounds__(kThreads) k_elementwise(int len, const Epi epi)
 {
+    begin_dependents();
+    wait_prerequisites();
     Acc<Epi::NRED> acc;
     epi.init(acc);
     for (int i = blockIdx.x * kThreads + threadIdx.x; i < len; i += gridDim.x * kThreads) epi.row(i, 0.0, acc);
-    epi.extra(acc);
+    epi.extra(acc, blockIdx.x, gridDim.x);
     if constexpr (Epi::NRED > 0) {
         int ops[Epi::NRED > 0 ? Epi::NRED : 1];
         epi.ops(ops);
@@ -530,9 +589,25 @@ inline int choose_staged(const std::vector<int> &rp, const std::vector<int> &ci)
     return pairs > 0 && 2 * runs >= pairs;
 }
 
-// Warp tiles: consecutive rows, at most kTileRows rows and kTileCap
-// entries; a row longer than kTileCap becomes kChunk-entry chunks.
-inline void build_tile_plan(const std::vector<int> &rp, TilePlan &p)
+// Entries per warp tile: a warp works through its tile one 256-entry window
+// after the other, each about 1 us of dependent loads, so a matrix of few
+// tiles is cut finer, down to one window a tile (nnz 1.2e5: 12.8 -> 10.3 us
+// out of cold caches).  Not where the tiles reach an eighth of the warps the
+// GPU holds at once: the next window's loads hide behind the current one's,
+// and short tiles have none (nnz 2e6, rows of 10: 20.9 us with 1024 entries a
+// tile, 24.8 with 256).
+inline int tile_cap(size_t nnz, int sms)
+{
+    const size_t warps = (size_t)sms * HPR_SPMV_MIN_BLOCKS * kWarps;
+    int cap = kTileCap;
+    while (cap > kSpmvWin && 8 * nnz < warps * (size_t)cap) cap /= 2;
+    return cap;
+}
+
+// Warp tiles: consecutive rows, at most kTileRows rows and `cap` entries
+// (a row longer than cap, up to kTileCap, is a tile of its own); a row longer
+// than kTileCap becomes kChunk-entry chunks.
+inline void build_tile_plan(const std::vector<int> &rp, TilePlan &p, int cap = kTileCap)
 {
     p = TilePlan();
     const int nrow = (int)rp.size() - 1;
@@ -551,7 +626,7 @@ inline void build_tile_plan(const std::vector<int> &rp, TilePlan &p)
         int r1 = r, nnz = 0;
         while (r1 < nrow && r1 - r < kTileRows) {
             const int l = rp[r1 + 1] - rp[r1];
-            if (l > kTileCap || (nnz + l > kTileCap && r1 > r)) break;
+            if (l > kTileCap || (nnz + l > cap && r1 > r)) break;
             nnz += l;
             ++r1;
         }

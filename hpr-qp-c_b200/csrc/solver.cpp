@@ -13,6 +13,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <chrono>
 #include <climits>
 #include <cmath>
@@ -58,6 +59,21 @@ int should_check_next(const HPRQPParams *p, const HPRQPRestart *r, size_t next)
     if (p->print_frequency > 0 && next % (size_t)p->print_frequency == 0) t = 1;
     return t;
 }
+
+// the first iteration after `iter` that the loop looks at: one on the check or
+// print grid, or the last one
+size_t next_event(const HPRQPParams *p, size_t iter)
+{
+    size_t nx = p->max_iter > iter ? p->max_iter : SIZE_MAX;
+    auto grid = [&](size_t d) { nx = std::min(nx, (iter / d + 1) * d); };
+    if (p->check_iter > 0) grid(p->check_iter);
+    if (p->print_frequency == -1) grid(adaptive_print_step(iter));
+    if (p->print_frequency > 0) grid((size_t)p->print_frequency);
+    return nx;
+}
+
+// iterations between two looks at the clock while none of them is checked
+constexpr size_t kMaxRun = 99;
 
 void restart_init(HPRQPRestart *r)
 {
@@ -357,6 +373,22 @@ HPRQPStatus hpr::solve_gpu_keep(const HPRQPModel *model, const HPRQPParams *para
         if (final_status != HPRQP_STATUS_CONTINUE) break;
 
         const int to_check = should_check_next(params, &rst, iter + 1);
+        if (!to_check) {
+            // nothing happens on the host before iteration `stop`: its steps
+            // but the last are launched together
+            const size_t stop = std::min(next_event(params, iter), iter + 1 + kMaxRun);
+            if (stop > iter + 1) {
+                const size_t run = stop - 1 - iter;
+                st = hpr::engine_partial_steps(eng, run);
+                if (st != HPRQP_STATUS_OK) {
+                    ret = st;
+                    goto done;
+                }
+                rst.inner += run;
+                iter += run - 1;  // (the loop adds one)
+                continue;
+            }
+        }
         st = hpr::engine_iteration_step(eng, rst.inner, to_check);
         if (st != HPRQP_STATUS_OK) {
             ret = st;

@@ -1,0 +1,63 @@
+"""Products with long rows in one launch, finer tiles, and the one-pass step of
+a diagonal Q (engine.cu, rowblock.cuh)."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n_long", [0, 1, 255, 256, 257])
+def test_long_rows_beside_tiles(engine_lib, n_long):
+    """Rows of more than 1024 entries among short and empty ones: up to 256 of
+    them are finished by the last chunk CTA, more by a kernel of their own.
+    Tolerance: 64-bit sums of len entries, 2 len eps sum |a_ij x_j|."""
+    import scipy.sparse as sp
+
+    rng = np.random.default_rng(n_long)
+    ncol = 3000
+    lens = np.concatenate([np.full(n_long, 1025) + rng.integers(0, 1100, n_long), rng.integers(0, 40, 700)])
+    rng.shuffle(lens)
+    indptr = np.concatenate([[0], np.cumsum(lens)])
+    indices = np.concatenate([np.sort(rng.choice(ncol, l, replace=False)) for l in lens]).astype(np.int64)
+    data = rng.standard_normal(len(indices))
+    x = rng.standard_normal(ncol)
+    M = sp.csr_matrix((data, indices, indptr), shape=(len(lens), ncol))
+    scale = abs(M) @ abs(x)
+    for _ in range(2):  # a second launch finds the chunk counter as the first did
+        y, _ = engine_lib.spmv(indptr, indices, data, ncol, x, reps=2)
+        assert np.all(np.abs(y - M @ x) <= 2 * np.finfo(float).eps * np.maximum(lens, 1) * scale)
+
+
+@pytest.mark.parametrize("n", [1, 31, 1000, 40001])
+def test_diagonal_step_equals_general_step(engine_lib, n):
+    """A Q of its diagonal alone against the same Q with stored zeros beside
+    it, which takes the two products: the same iterates, bit for bit (zeros
+    add nothing to a row's sum, and no reduction enters the first steps)."""
+    from hprqp import instances
+
+    inst = instances.plain_qp(5, n=max(n, 2), m=max(1, n // 3), a_density=min(0.3, 6.0 / n), m_rows=1, m_density=0.1,
+                              n_eq=0)
+    n = inst.n
+    d = np.random.default_rng(n).uniform(0.1, 2.0, n)
+    plain = instances.CSR(n, n, np.arange(n + 1), np.arange(n), d)
+    rows = np.repeat(np.arange(n), 2)
+    cols = np.stack([np.arange(n), (np.arange(n) + 1) % n], 1)
+    vals = np.stack([d, np.zeros(n)], 1)
+    o = np.argsort(cols, axis=1)
+    padded = instances.CSR(n, n, 2 * np.arange(n + 1), np.take_along_axis(cols, o, 1).ravel(),
+                           np.take_along_axis(vals, o, 1).ravel())
+    assert len(rows) == padded.nnz
+    old = engine_lib.set_single_cta_max_work(0)  # the device-wide engine
+    try:
+        got = []
+        for Q in (plain, padded):
+            inst.Q = Q
+            r = engine_lib.optimize(engine_lib.build_from_instance(inst),
+                                    engine_lib.Parameters(verbose=False, stoptol=1e-30, max_iter=57), as_numpy=True)
+            got.append(r)
+        for f in ("x", "y", "z", "w"):
+            np.testing.assert_array_equal(getattr(got[0], f), getattr(got[1], f), err_msg=f)
+    finally:
+        engine_lib.set_single_cta_max_work(old)
