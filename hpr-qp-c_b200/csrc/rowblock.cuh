@@ -595,12 +595,14 @@ inline int choose_staged(const std::vector<int> &rp, const std::vector<int> &ci)
 // out of cold caches).  Not where the tiles reach an eighth of the warps the
 // GPU holds at once: the next window's loads hide behind the current one's,
 // and short tiles have none (nnz 2e6, rows of 10: 20.9 us with 1024 entries a
-// tile, 24.8 with 256).
-inline int tile_cap(size_t nnz, int sms)
+// tile, 24.8 with 256).  k_spmv_staged works longer on a window, so that its
+// line lies at half of the warps (7.3e6 entries: 32.8 us with 1024, 43 with
+// 256; a portfolio QP with 1.2e6: 36 us a step with 256, 42 with 1024).
+inline int tile_cap(size_t nnz, int sms, bool staged)
 {
     const size_t warps = (size_t)sms * HPR_SPMV_MIN_BLOCKS * kWarps;
     int cap = kTileCap;
-    while (cap > kSpmvWin && 8 * nnz < warps * (size_t)cap) cap /= 2;
+    while (cap > kSpmvWin && (staged ? 2 : 8) * nnz < warps * (size_t)cap) cap /= 2;
     return cap;
 }
 
