@@ -862,75 +862,103 @@ __device__ __forceinline__ double row_absreduce(const int *rp, const double *v, 
     return sum ? warp_sum(acc) : warp_max(acc);
 }
 
-// column factors: sqrt of max/sum |.| over A' row j and Q row j
-// (reference gpu_compute_row_{max,sum}_abs_with_q_kernel, scale.cu:15-90)
-__global__ void k_col_factors(const DState S, int use_sum, double *cf)
+// Scaling factors of one pass.  Columns: sqrt of max/sum |.| over A' row j and
+// Q row j (reference gpu_compute_row_{max,sum}_abs_with_q_kernel,
+// scale.cu:15-90); rows: the same over A row r.  One warp per row; a long row
+// of A (its chunks hold it) takes one warp per chunk where a maximum is asked
+// for, k_long_factors ends it.  Sums keep one warp per row: their order.
+__global__ void k_factors(const DState S, int use_sum, double *cf, double *rf)
 {
     const int lane = threadIdx.x & 31;
     const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int j = wid; j < S.n; j += nw) {
-        double a = S.m > 0 ? row_absreduce(S.AT.rp, S.AT.v, j, lane, use_sum) : 0.0;
-        const double b = row_absreduce(S.Q.rp, S.Q.v, j, lane, use_sum);
-        a = use_sum ? a + b : fmax(a, b);
-        if (lane == 0) cf[j] = a > 0.0 ? sqrt(a) : 1.0;
+    const int chunks = use_sum ? 0 : S.A.nchunks;
+    for (int it = wid; it < chunks + S.m + S.n; it += nw) {
+        if (it < chunks) {  // first: the longest items
+            const int4 C = S.A.chunks[it];
+            double a = 0.0;
+            for (int k = C.y + lane; k < C.z; k += 32) a = fmax(a, fabs(S.A.v[k]));
+            a = warp_max(a);
+            if (lane == 0) S.A.chunk_partial[C.w] = a;
+        } else if (it < chunks + S.m) {
+            const int r = it - chunks;
+            if (!use_sum && S.A.rp[r + 1] - S.A.rp[r] > kTileCap) continue;
+            const double a = row_absreduce(S.A.rp, S.A.v, r, lane, use_sum);
+            if (lane == 0) rf[r] = a > 0.0 ? sqrt(a) : 1.0;
+        } else {
+            const int j = it - chunks - S.m;
+            double a = S.m > 0 ? row_absreduce(S.AT.rp, S.AT.v, j, lane, use_sum) : 0.0;
+            const double b = row_absreduce(S.Q.rp, S.Q.v, j, lane, use_sum);
+            a = use_sum ? a + b : fmax(a, b);
+            if (lane == 0) cf[j] = a > 0.0 ? sqrt(a) : 1.0;
+        }
     }
 }
 
-__global__ void k_row_factors(const DState S, int use_sum, double *rf)
+__global__ void k_long_factors(const DCsr A, double *rf)
 {
-    const int lane = threadIdx.x & 31;
-    const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int r = wid; r < S.m; r += nw) {
-        const double a = row_absreduce(S.A.rp, S.A.v, r, lane, use_sum);
-        if (lane == 0) rf[r] = a > 0.0 ? sqrt(a) : 1.0;
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.nlong; i += gridDim.x * blockDim.x) {
+        const int2 lr = A.long_rows[i];
+        const int c1 = i + 1 < A.nlong ? A.long_rows[i + 1].y : A.nchunks;
+        double a = 0.0;
+        for (int c = lr.y; c < c1; ++c) a = fmax(a, A.chunk_partial[c]);
+        rf[lr.x] = a > 0.0 ? sqrt(a) : 1.0;
     }
 }
 
 // scale rows of M by 1/rs[row] (multiplication by the reciprocal), then
 // columns by division with cs[col]; same two roundings as the reference's
 // gpu_scale_rows_csr_kernel + gpu_scale_cols_csr_kernel (scale.cu:113-150)
-__device__ __forceinline__ void scale_row(const DCsr &M, int r, int lane, const double *rs, const double *cs)
+__device__ __forceinline__ void scale_entries(const DCsr &M, int r, int k0, int k1, int lane, const double *rs,
+                                              const double *cs)
 {
     const double inv = 1.0 / rs[r];
-    for (int k = M.rp[r] + lane; k < M.rp[r + 1]; k += 32) {
+    for (int k = k0 + lane; k < k1; k += 32) {
         double v = M.v[k] * inv;
         v /= cs[M.ci[k]];
         M.v[k] = v;
     }
 }
 
-__global__ void k_apply_n(const DState S, const double *cf, const double *rf)
+// item `it` of the nrow + nchunks items of a matrix: a chunk of a long row
+// (first: the longest), or a row that is not long
+__device__ __forceinline__ void scale_item(const DCsr &M, int it, int lane, const double *rs, const double *cs)
 {
-    const int lane = threadIdx.x & 31;
-    const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int j = wid; j < S.n; j += nw) {
-        scale_row(S.Q, j, lane, cf, cf);
-        if (S.m > 0) scale_row(S.AT, j, lane, cf, rf);
-        if (lane == 0) {
-            S.col_norm[j] *= cf[j];
-            S.c[j] /= cf[j];
-            S.l[j] *= cf[j];
-            S.u[j] *= cf[j];
-        }
+    if (it < M.nchunks) {
+        const int4 C = M.chunks[it];
+        scale_entries(M, C.x, C.y, C.z, lane, rs, cs);
+    } else {
+        const int r = it - M.nchunks, k0 = M.rp[r], k1 = M.rp[r + 1];
+        if (k1 - k0 <= kTileCap) scale_entries(M, r, k0, k1, lane, rs, cs);
     }
 }
 
-__global__ void k_apply_m(const DState S, const double *cf, const double *rf)
+// One scaling pass applied: the three matrices by warps, the vectors by
+// threads.  With one warp per row the 120 rows of 60,000 entries of a
+// portfolio QP took 1.35 ms a pass (a division and a gather after the other);
+// by chunks of 1024 entries a whole pass takes 0.17 ms.
+__global__ void k_apply(const DState S, const double *cf, const double *rf)
 {
-    const int lane = threadIdx.x & 31;
-    const int wid = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int nw = (gridDim.x * blockDim.x) >> 5;
-    for (int r = wid; r < S.m; r += nw) {
-        scale_row(S.A, r, lane, rf, cf);
-        if (lane == 0) {
-            S.row_norm[r] *= rf[r];
-            S.AL[r] /= rf[r];
-            S.AU[r] /= rf[r];
-            if (S.rhs) S.rhs[r] /= rf[r];
-        }
+    const int tid = blockIdx.x * blockDim.x + threadIdx.x, nth = gridDim.x * blockDim.x;
+    const int lane = threadIdx.x & 31, wid = tid >> 5, nw = nth >> 5;
+    const int items_a = S.m > 0 ? S.A.nchunks + S.m : 0, items_at = S.m > 0 ? S.AT.nchunks + S.n : 0;
+    const int items = items_a + items_at + S.Q.nchunks + S.n;
+    for (int it = wid; it < items; it += nw) {
+        if (it < items_a) scale_item(S.A, it, lane, rf, cf);
+        else if (it < items_a + items_at) scale_item(S.AT, it - items_a, lane, cf, rf);
+        else scale_item(S.Q, it - items_a - items_at, lane, cf, cf);
+    }
+    for (int j = tid; j < S.n; j += nth) {
+        S.col_norm[j] *= cf[j];
+        S.c[j] /= cf[j];
+        S.l[j] *= cf[j];
+        S.u[j] *= cf[j];
+    }
+    for (int r = tid; r < S.m; r += nth) {
+        S.row_norm[r] *= rf[r];
+        S.AL[r] /= rf[r];
+        S.AU[r] /= rf[r];
+        if (S.rhs) S.rhs[r] /= rf[r];
     }
 }
 
@@ -1459,10 +1487,10 @@ HPRQPStatus engine_create(const HPRQPModel *model, const HPRQPParams *params, En
         const int wgrid = std::max(1, std::min((int)((nmax * 32 + kThreads - 1) / kThreads), e->num_sms * 8));
         for (int pass = 0; pass < 11; ++pass) {
             const int use_sum = pass == 10;
-            k_col_factors<<<wgrid, kThreads, 0, e->stream>>>(S, use_sum, S.fac_c);
+            k_factors<<<wgrid, kThreads, 0, e->stream>>>(S, use_sum, S.fac_c, S.fac_r);
             count_launch();
-            if (m > 0) {
-                k_row_factors<<<wgrid, kThreads, 0, e->stream>>>(S, use_sum, S.fac_r);
+            if (S.A.nlong && !use_sum) {
+                k_long_factors<<<(S.A.nlong + kThreads - 1) / kThreads, kThreads, 0, e->stream>>>(S.A, S.fac_r);
                 count_launch();
             }
             if (S.nvc) {
@@ -1473,12 +1501,8 @@ HPRQPStatus engine_create(const HPRQPModel *model, const HPRQPParams *params, En
                 k_cone_block_max<<<wgrid, kThreads, 0, e->stream>>>(S.fac_r, S.rco, S.nrc);
                 count_launch();
             }
-            k_apply_n<<<wgrid, kThreads, 0, e->stream>>>(S, S.fac_c, S.fac_r);
+            k_apply<<<wgrid, kThreads, 0, e->stream>>>(S, S.fac_c, S.fac_r);
             count_launch();
-            if (m > 0) {
-                k_apply_m<<<wgrid, kThreads, 0, e->stream>>>(S, S.fac_c, S.fac_r);
-                count_launch();
-            }
         }
         E_CK(cudaGetLastError());
     }

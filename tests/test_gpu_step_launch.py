@@ -61,3 +61,40 @@ def test_diagonal_step_equals_general_step(engine_lib, n):
             np.testing.assert_array_equal(getattr(got[0], f), getattr(got[1], f), err_msg=f)
     finally:
         engine_lib.set_single_cta_max_work(old)
+
+
+@pytest.mark.parametrize("n", [1025, 2100])
+def test_scaling_of_long_rows(engine_lib, n):
+    """Ruiz x10 and Pock-Chambolle with rows longer than a chunk, against the
+    same passes in numpy.  Each of the 11 passes rounds a value three times,
+    the last one's sums have chains of at most n / 32 + 5 additions: 35 + 2 *
+    71 eps, taken as 200."""
+    import scipy.sparse as sp
+    from hprqp import instances
+
+    rng = np.random.default_rng(n)
+    inst = instances.plain_qp(3, n=n, m=40, a_density=0.01, m_rows=30, m_density=0.02, n_eq=10)
+    A = inst.A.to_scipy().tolil()
+    A[0, :] = rng.standard_normal(n)
+    A[7, : n - 1] = 10.0 * rng.standard_normal(n - 1)
+    A = A.tocsr()
+    A.sort_indices()
+    inst.A = instances.CSR(40, n, A.indptr.astype(np.int64), A.indices.astype(np.int64), A.data)
+    model = engine_lib.build_from_instance(inst)
+    got = engine_lib.setup_info(model, dump=True)
+    arrays = engine_lib.model_arrays(model)
+    Q, A = (sp.csr_matrix((arrays[k + "_data"], arrays[k + "_indices"], arrays[k + "_indptr"]), shape=(r, n)).toarray()
+            for k, r in (("q", n), ("a", arrays["m"])))
+    rows = np.repeat(np.arange(arrays["m"]), np.diff(arrays["a_indptr"]))
+    rn, cn = np.ones(A.shape[0]), np.ones(n)
+    for p in range(11):
+        if p < 10:
+            rf, cf = abs(A).max(1), np.maximum(abs(A).max(0), abs(Q).max(0))
+        else:
+            rf, cf = abs(A).sum(1), abs(A).sum(0) + abs(Q).sum(0)
+        rf, cf = np.sqrt(np.where(rf > 0, rf, 1.0)), np.sqrt(np.where(cf > 0, cf, 1.0))
+        A, Q = A / rf[:, None] / cf, Q / cf[:, None] / cf
+        rn, cn = rn * rf, cn * cf
+    np.testing.assert_allclose(got["row_norm"], rn, rtol=200 * np.finfo(float).eps)
+    np.testing.assert_allclose(got["col_norm"], cn, rtol=200 * np.finfo(float).eps)
+    np.testing.assert_allclose(got["a_val"], A[rows, arrays["a_indices"]], rtol=200 * np.finfo(float).eps)
