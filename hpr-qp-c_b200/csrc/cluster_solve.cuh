@@ -114,10 +114,10 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve(const ClusterAr
 #pragma unroll
     for (int r = 0; r < C; ++r) far[r] = MULTI ? cl_map(cl_smem(sm), r) - cl_smem(sm) : 0u;
     auto sync = [&]() {
+        // (not the .aligned forms: they need a converged warp, which code before
+        // a barrier does not promise; a diverged one would arrive in parts)
         __syncwarp();
-        if (MULTI)
-            asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::
-                             : "memory");
+        if (MULTI) asm volatile("barrier.cluster.arrive.release;\n\tbarrier.cluster.wait.acquire;" ::: "memory");
         else __syncthreads();
     };
     // store to the same shared address of every CTA of the cluster
