@@ -28,6 +28,7 @@
 #include "hprqp.h"
 #include "batch_device.cuh"
 #include "cluster_solve.h"
+#include "pool.h"
 #include "rowblock.cuh"
 
 #include <cuda_runtime.h>
@@ -1400,8 +1401,8 @@ static HPRQPStatus balloc(HPRQPBatch *b, T **p, size_t count)
 {
     *p = nullptr;
     if (count == 0) count = 1;
-    void *ptr = nullptr;
-    if (cudaMalloc(&ptr, count * sizeof(T)) != cudaSuccess) {
+    void *ptr = pool_alloc(count * sizeof(T));
+    if (!ptr) {
         fprintf(stderr, "hprqp-b200 batch: cudaMalloc(%zu bytes) failed\n", count * sizeof(T));
         return HPRQP_STATUS_ALLOCATION_FAILED;
     }
@@ -1443,16 +1444,22 @@ private:
 
 static void batch_free(HPRQPBatch *b)
 {
-    for (void *p : b->allocs) cudaFree(p);
+    int current = -1;
+    cudaGetDevice(&current);
+    if (current != b->device) cudaSetDevice(b->device);
+    if (b->stream) cudaStreamSynchronize(b->stream);
+    for (auto &st : b->side) cudaStreamSynchronize(st);
+    for (void *p : b->allocs) pool_free(p);
     b->allocs.clear();
-    if (b->h_abort) cudaFreeHost(b->h_abort);
+    pool_pinned_return(b->h_abort);
     b->h_abort = b->d_abort = nullptr;
     for (auto &m : b->models) model_free(&m);
     b->models.clear();
-    if (b->stream) cudaStreamDestroy(b->stream);
-    for (auto &st : b->side) cudaStreamDestroy(st);
+    pool_stream_return(b->stream);
+    for (auto &st : b->side) pool_stream_return(st);
     b->side.clear();
     b->stream = nullptr;
+    if (current >= 0 && current != b->device) cudaSetDevice(current);
 }
 
 // The per-instance SpMV autotuner: the lane-group width of cta_spmv for one
@@ -2052,7 +2059,7 @@ static HPRQPStatus batch_create_impl(size_t K, const size_t *var_offsets, const 
     };
     if (cudaSetDevice(device_number) != cudaSuccess ||
         cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, device_number) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess)
+        !(b->stream = pool_stream()))
         return fail(HPRQP_STATUS_NOT_IMPLEMENTED);
     BatchArgs &G = b->args;
     G.K = (int)K;
@@ -2097,8 +2104,7 @@ static HPRQPStatus batch_create_impl(size_t K, const size_t *var_offsets, const 
     // the abort flag (host-mapped memory) exists only for batches a caller
     // holds a handle to: the one-call forms cannot be asked to stop
     if (abortable) {
-        if (cudaHostAlloc((void **)&b->h_abort, sizeof(int), cudaHostAllocMapped) != cudaSuccess ||
-            cudaHostGetDevicePointer((void **)&b->d_abort, b->h_abort, 0) != cudaSuccess)
+        if (!(b->h_abort = (int *)pool_pinned((void **)&b->d_abort)))
             return fail(HPRQP_STATUS_NOT_IMPLEMENTED);
         __atomic_store_n(b->h_abort, 0, __ATOMIC_SEQ_CST);
     }
@@ -2176,8 +2182,8 @@ static HPRQPStatus phase_launch(HPRQPBatch *b, SolveLaunch &L, const int *order,
         return bt == kBigCta ? k_batch_solve<kBigCta> : bt == kMidCta ? k_batch_solve<kMidCta> : k_batch_solve<kSmallCta>;
     };
     while ((int)b->side.size() + 1 < ns) {
-        cudaStream_t st = nullptr;
-        B_CK(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+        cudaStream_t st = pool_stream();
+        if (!st) return HPRQP_STATUS_NOT_IMPLEMENTED;
         b->side.push_back(st);
     }
     int vec_smem[kMaxGroups] = {}, slots = 0, off[kMaxGroups] = {}, ctas = 0, coff[kMaxGroups] = {};

@@ -8,6 +8,7 @@
 // Halpern counter) live in a small device struct so the step can be captured
 // once in a CUDA graph and replayed.
 #include "engine.h"
+#include "pool.h"
 #include "rowblock.cuh"
 
 #include <cooperative_groups.h>
@@ -1075,6 +1076,7 @@ __global__ void __launch_bounds__(kThreads) k_golden_diag(const DState S, double
 struct HostOut {
     double v[64];
 };
+static_assert(sizeof(HostOut) <= kPinnedBytes, "the pool's pinned words hold it");
 
 // partials up to which every CTA of a kernel folds them itself
 constexpr int kFoldBlocks = 1024;
@@ -1105,11 +1107,9 @@ static HPRQPStatus dalloc(Engine *e, T **p, size_t count)
 {
     *p = nullptr;
     if (count == 0) count = 1;
-    void *ptr = nullptr;
-    cudaError_t err = cudaMalloc(&ptr, count * sizeof(T));
-    if (err != cudaSuccess) {
-        fprintf(stderr, "hprqp-b200: cudaMalloc(%zu bytes) failed: %s\n", count * sizeof(T),
-                cudaGetErrorString(err));
+    void *ptr = pool_alloc(count * sizeof(T));
+    if (!ptr) {
+        fprintf(stderr, "hprqp-b200: cudaMalloc(%zu bytes) failed\n", count * sizeof(T));
         return HPRQP_STATUS_ALLOCATION_FAILED;
     }
     e->allocs.push_back(ptr);
@@ -1332,10 +1332,15 @@ static void free_engine_memory(Engine *e)
 {
     for (auto &g : e->step_graph)
         if (g) cudaGraphExecDestroy(g);
-    for (void *p : e->allocs) cudaFree(p);
+    int current = -1;
+    cudaGetDevice(&current);
+    if (current != e->device) cudaSetDevice(e->device);
+    if (e->stream) cudaStreamSynchronize(e->stream);
+    for (void *p : e->allocs) pool_free(p);
     e->allocs.clear();
-    if (e->hout) cudaFreeHost(e->hout);
-    if (e->stream) cudaStreamDestroy(e->stream);
+    pool_pinned_return(e->hout);
+    pool_stream_return(e->stream);
+    if (current >= 0 && current != e->device) cudaSetDevice(current);
 }
 
 void engine_destroy(Engine *e)
@@ -1380,10 +1385,10 @@ HPRQPStatus engine_create(const HPRQPModel *model, const HPRQPParams *params, En
     HPR_TRACE("create: set device");
     E_CK(cudaSetDevice(e->device));
     E_CK(cudaDeviceGetAttribute(&e->num_sms, cudaDevAttrMultiProcessorCount, e->device));
-    E_CK(cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking));
-    E_CK(cudaHostAlloc((void **)&e->hout, sizeof(HostOut), cudaHostAllocMapped));
-    E_CK(cudaHostGetDevicePointer((void **)&e->dout, e->hout, 0));
-    memset(e->hout, 0, sizeof(HostOut));
+    if (!(e->stream = pool_stream()) || !(e->hout = (HostOut *)pool_pinned((void **)&e->dout))) {
+        engine_destroy(e);
+        return HPRQP_STATUS_NOT_IMPLEMENTED;
+    }
 
     HPR_TRACE("create: host alloc ok");
     DState &S = e->S;
@@ -2469,7 +2474,7 @@ static HPRQPStatus spmv_standalone(size_t nrow, size_t ncol, size_t nnz, const s
         engine_destroy(e);
         return s;
     };
-    if (cudaStreamCreateWithFlags(&e->stream, cudaStreamNonBlocking) != cudaSuccess)
+    if (cudaGetDevice(&e->device) != cudaSuccess || !(e->stream = pool_stream()))
         return fail(HPRQP_STATUS_NOT_IMPLEMENTED);
     HPRQPMatrixCSR h;
     h.nrow = nrow;

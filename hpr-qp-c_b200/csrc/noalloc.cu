@@ -31,6 +31,7 @@
 // The call selects `device` for its own work and restores the caller's
 // current device before it returns, on every path.
 #include "hprqp_b200.h"
+#include "pool.h"
 #include "rowblock.cuh"
 
 #include <cuda.h>
@@ -39,6 +40,38 @@
 #include <cmath>
 #include <cstdio>
 #include <mutex>
+
+namespace hpr {
+
+// Identity of the current context (cuCtxGetId, reached through the runtime's
+// driver entry points so the library links only cudart); false when the
+// driver does not offer it.
+bool current_context_id(unsigned long long *id)
+{
+    using GetCurrentFn = CUresult (*)(CUcontext *);
+    using GetIdFn = CUresult (*)(CUcontext, unsigned long long *);
+    static GetCurrentFn get_current = nullptr;
+    static GetIdFn get_id = nullptr;
+    static bool looked_up = false;
+    if (!looked_up) {
+        void *f0 = nullptr, *f1 = nullptr;
+        cudaDriverEntryPointQueryResult q0, q1;
+        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f0, cudaEnableDefault, &q0) == cudaSuccess &&
+            q0 == cudaDriverEntryPointSuccess && cudaGetDriverEntryPoint("cuCtxGetId", &f1, cudaEnableDefault, &q1) ==
+                                                     cudaSuccess && q1 == cudaDriverEntryPointSuccess) {
+            get_current = (GetCurrentFn)f0;
+            get_id = (GetIdFn)f1;
+        }
+        cudaGetLastError();  // a missing entry point is not an error of this call
+        looked_up = true;
+    }
+    if (!get_current || !get_id) return false;
+    CUcontext ctx = nullptr;
+    if (get_current(&ctx) != CUDA_SUCCESS || ctx == nullptr) return false;
+    return get_id(ctx, id) == CUDA_SUCCESS;
+}
+
+}  // namespace hpr
 
 namespace hpr_noalloc {
 
@@ -167,33 +200,7 @@ static int grid_for(long long work)
     return (int)(g < 1 ? 1 : (g > kMaxBlocks ? kMaxBlocks : g));
 }
 
-// Identity of the current context (cuCtxGetId, reached through the runtime's
-// driver entry points so the library links only cudart); false when the
-// driver does not offer it.
-static bool current_context_id(unsigned long long *id)
-{
-    using GetCurrentFn = CUresult (*)(CUcontext *);
-    using GetIdFn = CUresult (*)(CUcontext, unsigned long long *);
-    static GetCurrentFn get_current = nullptr;
-    static GetIdFn get_id = nullptr;
-    static bool looked_up = false;
-    if (!looked_up) {
-        void *f0 = nullptr, *f1 = nullptr;
-        cudaDriverEntryPointQueryResult q0, q1;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f0, cudaEnableDefault, &q0) == cudaSuccess &&
-            q0 == cudaDriverEntryPointSuccess && cudaGetDriverEntryPoint("cuCtxGetId", &f1, cudaEnableDefault, &q1) ==
-                                                     cudaSuccess && q1 == cudaDriverEntryPointSuccess) {
-            get_current = (GetCurrentFn)f0;
-            get_id = (GetIdFn)f1;
-        }
-        cudaGetLastError();  // a missing entry point is not an error of this call
-        looked_up = true;
-    }
-    if (!get_current || !get_id) return false;
-    CUcontext ctx = nullptr;
-    if (get_current(&ctx) != CUDA_SUCCESS || ctx == nullptr) return false;
-    return get_id(ctx, id) == CUDA_SUCCESS;
-}
+using hpr::current_context_id;
 
 // Address of the scratch array on `device`, which must be current: looked up
 // on the first call in each context of the device and cached with that
