@@ -1579,11 +1579,11 @@ static size_t cluster_smem_limit()
     return 227 * 1024 - 8 * 1024;  // 8 KB for its static shared memory
 }
 
-static void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int C, int grid, size_t smem,
-                           cudaStream_t stream)
+static void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int C, bool resident, int grid,
+                           size_t smem, cudaStream_t stream)
 {
     cfg.gridDim = dim3(grid);
-    cfg.blockDim = dim3(kClThreads);
+    cfg.blockDim = dim3(cluster_threads(C, resident));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = stream;
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -1670,7 +1670,7 @@ static int max_clusters(int device, int sms, int C)
     const size_t smem = cluster_smem_limit();
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
-    cluster_config(cfg, at, C, C, smem, nullptr);
+    cluster_config(cfg, at, C, true, C, smem, nullptr);
     int c = 0;
     if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
         (C > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
@@ -1798,10 +1798,11 @@ static void make_groups(const HPRQPBatch *b, const std::vector<int> &ids, const 
 
 // The first phase of a solve.  Batches of at most one instance per SM: all
 // run at once, SMs spread by choose_clusters.  Larger ones: one CTA per
-// instance, the kMidCta instances (mid_cta_instance) in a launch started
-// first, so that every small instance -- whose iteration counts vary most --
-// starts at once, and the others in a launch whose CTAs take the SMs as the
-// first one's finish.  On entry order holds all instances, largest first; on
+// instance, the kMidCta instances (mid_cta_instance) in launches started
+// first -- those that a CTA's shared memory holds in k_cluster_solve's
+// one-CTA form -- so that the small instances, whose iteration counts vary
+// most, start at once, and the others in a launch whose CTAs take the SMs as
+// the first ones' finish.  On entry order holds all instances, largest first; on
 // return its first half is cut into b->groups.
 static HPRQPStatus first_phase(HPRQPBatch *b, std::vector<int> &order)
 {
@@ -1812,6 +1813,12 @@ static HPRQPStatus first_phase(HPRQPBatch *b, std::vector<int> &order)
         std::vector<Item> items(K);
         for (size_t e = 0; e < K; ++e) items[e] = {b, (size_t)ids[e]};
         if (!choose_clusters(items, true, C)) return HPRQP_STATUS_NOT_IMPLEMENTED;
+    } else if (b->cta_threads == kBigCta) {
+        for (size_t e = 0; e < K; ++e) {
+            const size_t k = (size_t)ids[e];
+            C[e] = instance_vw(b, k) == kMidCta / 32 && cluster_fits(b, k, 1) && cluster_resident(b, k, 1) &&
+                   iteration_us(b, k, 1) < iteration_us(b, k, 0);
+        }
     }
     make_groups(b, ids, C, pos, b->groups);
     for (size_t e = 0; e < K; ++e) order[e] = ids[pos[e]];
@@ -2227,6 +2234,11 @@ static HPRQPStatus phase_launch(HPRQPBatch *b, SolveLaunch &L, const int *order,
         vec_smem[s] = HPR_BATCH_VEC_SMEM && vec_bytes <= smem_limit(bt) && pool_per_sm <= kPoolPerSm;
         smem[s] = vec_smem[s] ? vec_bytes : 0;
         B_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[s]));
+        // an SM that ran a cluster's CTA keeps its carveout (28 KB of L1) unless
+        // it is told otherwise: 400 QPs beside the launch of the small ones
+        // 455 ms without this line, 298 with it
+        B_CK(cudaFuncSetAttribute(kern, cudaFuncAttributePreferredSharedMemoryCarveout,
+                                  (int)std::min<size_t>(100, (100 * pool_per_sm * vec_smem[s] + 228 * 1024 - 1) / (228 * 1024))));
         int per_sm = 0;
         B_CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, bt, smem[s]));
         L.grid[s] = std::max(1, std::min((int)g.count, b->num_sms * std::max(per_sm, 1)));
@@ -2314,7 +2326,7 @@ static HPRQPStatus phase_launch(HPRQPBatch *b, SolveLaunch &L, const int *order,
             P.smem_bytes = (int)smem[s];
             cudaLaunchConfig_t cfg = {};
             cudaLaunchAttribute at[1];
-            cluster_config(cfg, at, g.C, L.grid[s], smem[s], stream);
+            cluster_config(cfg, at, g.C, res[s], L.grid[s], smem[s], stream);
             err = cluster_launch_of(g.C, res[s], cfg, P);
         } else {
             kern_of(32 * g.vw)<<<L.grid[s], 32 * g.vw, smem[s], stream>>>(A);

@@ -27,7 +27,8 @@
 // on one SM, 230 SM-us on 8), so clusters serve the batches that leave SMs
 // idle and the last instances of the others (choose_clusters, batch_launch).
 // 256 threads: 512 are slower (128 registers spill, and a CTA's few rows on
-// twice the warps cost issue slots: n = 1000 on 8 CTAs 7.0 against 13.5 ms).
+// twice the warps cost issue slots: n = 1000 on 8 CTAs 7.0 against 13.5 ms),
+// except where one CTA holds all of an instance's rows (cluster_threads).
 //
 // Results equal k_batch_solve's bit for bit.  A row's sum depends on the
 // lane-group width only.  Reductions are folded in that kernel's order: the
@@ -45,7 +46,6 @@
 
 namespace hpr {
 
-constexpr int kClWarps = kClThreads / 32;
 // places in an own row's record
 enum { kX, kW, kLx, kLw, kAty, kLaty, kQw, kC, kL, kU, kXh };
 enum { kY, kLy, kAL, kAU, kYb };
@@ -89,10 +89,10 @@ struct CMat {
     double2 *gv;
 };
 
-template <int C, bool RES>
-__global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve(const ClusterArgs P)
+template <int C, bool RES, int NT>
+__global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
 {
-    constexpr int NT = kClThreads, NW = kClWarps;
+    constexpr int NW = NT / 32;
     constexpr bool MULTI = C > 1;
     extern __shared__ __align__(16) double sm[];
     __shared__ CtaState S;
@@ -1473,14 +1473,15 @@ __global__ void __launch_bounds__(kClThreads, 1) k_cluster_solve(const ClusterAr
 template <int C>
 const void *cluster_kernel(bool resident)
 {
-    return resident ? (const void *)k_cluster_solve<C, true> : (const void *)k_cluster_solve<C, false>;
+    return resident ? (const void *)k_cluster_solve<C, true, cluster_threads(C, true)>
+                    : (const void *)k_cluster_solve<C, false, cluster_threads(C, false)>;
 }
 
 template <int C>
 cudaError_t cluster_launch(bool resident, const cudaLaunchConfig_t &cfg, const ClusterArgs &P)
 {
-    return resident ? cudaLaunchKernelEx(&cfg, k_cluster_solve<C, true>, P)
-                    : cudaLaunchKernelEx(&cfg, k_cluster_solve<C, false>, P);
+    return resident ? cudaLaunchKernelEx(&cfg, k_cluster_solve<C, true, cluster_threads(C, true)>, P)
+                    : cudaLaunchKernelEx(&cfg, k_cluster_solve<C, false, cluster_threads(C, false)>, P);
 }
 
 }  // namespace hpr

@@ -7,7 +7,11 @@
 
 namespace hpr {
 
-constexpr int kClThreads = 256;
+// Threads of a CTA.  One CTA with a whole instance in its shared memory has
+// rows for more warps (us an iteration of n = 220 / 450 with all SMs busy:
+// 8.6 / 16.1 with 256 threads, 6.9 / 13.8 with 512, 12.2 / 17.7 in
+// k_batch_solve; n = 100: 4.6, 5.3, 7.9).
+__host__ __device__ constexpr int cluster_threads(int C, bool resident) { return C == 1 && resident ? 512 : 256; }
 constexpr int kClMaxLen = 8190;  // columns as 16-bit byte offsets, the zero entry included
 // doubles of shared memory per own row of an n- and an m-vector (odd: a warp's
 // rows fall on different banks)
