@@ -1813,10 +1813,10 @@ static HPRQPStatus first_phase(HPRQPBatch *b, std::vector<int> &order)
         std::vector<Item> items(K);
         for (size_t e = 0; e < K; ++e) items[e] = {b, (size_t)ids[e]};
         if (!choose_clusters(items, true, C)) return HPRQP_STATUS_NOT_IMPLEMENTED;
-    } else if (b->cta_threads == kBigCta) {
+    } else {
         for (size_t e = 0; e < K; ++e) {
             const size_t k = (size_t)ids[e];
-            C[e] = instance_vw(b, k) == kMidCta / 32 && cluster_fits(b, k, 1) && cluster_resident(b, k, 1) &&
+            C[e] = instance_vw(b, k) != kBigCta / 32 && cluster_fits(b, k, 1) && cluster_resident(b, k, 1) &&
                    iteration_us(b, k, 1) < iteration_us(b, k, 0);
         }
     }
