@@ -1203,6 +1203,24 @@ static void launch_rb_at(Engine *e, const DCsr &M, const double *x, Epi epi, siz
     if (M.grid_long > 1) launch_k(e, k_long_epi<Epi>, M.grid_long, M, epi);
 }
 
+// Independent products of two different matrices (a matrix's chunk partials
+// and their counter serve one product at a time), in one launch where neither
+// is staged nor leaves long rows to a second kernel.
+template <class Epi1, class Epi2>
+static void launch_rb2(Engine *e, const DCsr &M1, const double *x1, Epi1 epi1, size_t poff1, const DCsr &M2,
+                       const double *x2, Epi2 epi2, size_t poff2)
+{
+    if (M1.nrow == 0 || M2.nrow == 0 || M1.staged || M2.staged || M1.grid_long > 1 || M2.grid_long > 1) {
+        launch_rb_at(e, M1, x1, epi1, poff1);
+        launch_rb_at(e, M2, x2, epi2, poff2);
+        return;
+    }
+    epi1.partials = e->partials + poff1;
+    epi2.partials = e->partials + poff2;
+    launch_k(e, k_spmv2<Epi1, Epi2>, M1.grid_chunk + M1.grid_main + M2.grid_chunk + M2.grid_main, M1, x1, epi1, M2, x2,
+             epi2);
+}
+
 template <class Epi>
 static void launch_rb(Engine *e, const DCsr &M, const double *x, Epi epi)
 {
@@ -2266,12 +2284,11 @@ HPRQPStatus engine_adjoint(Engine *e, const double *gx, const double *gy, double
             if (m > 0) {
                 EpiStore q;
                 q.out = tmp;
-                launch_rb(e, S.Q, v, q);
                 EpiAdjM am;
                 am.yb = S.y_bar;
                 am.vm = v + n;
                 am.vnm = vn + n;
-                launch_rb_at(e, S.A, v, am, pa);
+                launch_rb2(e, S.Q, v, q, pl, S.A, v, am, pa);
                 fa[nf++] = spec_of<EpiAdjM>(S.A.npart(), 0, pa);
                 EpiAdjN an;
                 an.zb = S.z_bar;

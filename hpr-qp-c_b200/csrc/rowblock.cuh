@@ -301,11 +301,11 @@ __device__ __forceinline__ void long_rows(const DCsr &M, const Epi &epi, int cta
 // tiles run beside the chunks (portfolio QP, 120 rows of 60,000 entries and
 // 300 of 200: y = A x out of cold caches 44 us in three launches, 36 in one).
 template <class Epi>
-__device__ __forceinline__ void chunk_cta(const DCsr &M, const double *xin, const Epi &epi)
+__device__ __forceinline__ void chunk_cta(const DCsr &M, const double *xin, const Epi &epi, int bid)
 {
     __shared__ unsigned s_last;
     const int lane = threadIdx.x & 31;
-    const int c = blockIdx.x * kWarps + (threadIdx.x >> 5);
+    const int c = bid * kWarps + (threadIdx.x >> 5);
     int4 C = make_int4(0, 0, 0, 0);
     if (c < M.nchunks) C = M.chunks[c];
     wait_prerequisites();
@@ -327,15 +327,16 @@ __device__ __forceinline__ void chunk_cta(const DCsr &M, const double *xin, cons
     if (s_last) long_rows(M, epi, 0);
 }
 
+// CTA bid of a product (of its grid_chunk + grid_main)
 template <class Epi>
-__global__ void __launch_bounds__(kThreads, HPR_SPMV_MIN_BLOCKS) k_spmv(const DCsr M, const double *xin, const Epi epi)
+__device__ __forceinline__ void spmv_cta(const DCsr &M, const double *xin, const Epi &epi, int bid,
+                                         double (*s_row)[kTileRows])
 {
-    __shared__ double s_row[kWarps][kTileRows];
-    if ((int)blockIdx.x < M.grid_chunk) {
-        chunk_cta(M, xin, epi);
+    if (bid < M.grid_chunk) {
+        chunk_cta(M, xin, epi, bid);
         return;
     }
-    const int cta = blockIdx.x - M.grid_chunk;
+    const int cta = bid - M.grid_chunk;
     Acc<Epi::NRED> acc;
     epi.init(acc);
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -370,6 +371,27 @@ __global__ void __launch_bounds__(kThreads, HPR_SPMV_MIN_BLOCKS) k_spmv(const DC
         epi.ops(ops);
         block_reduce_store<Epi::NRED>(acc, ops, epi.partials + (size_t)cta * Epi::NRED);
     }
+}
+
+template <class Epi>
+__global__ void __launch_bounds__(kThreads, HPR_SPMV_MIN_BLOCKS) k_spmv(const DCsr M, const double *xin, const Epi epi)
+{
+    __shared__ double s_row[kWarps][kTileRows];
+    spmv_cta(M, xin, epi, blockIdx.x, s_row);
+}
+
+// Two products that do not depend on each other, side by side in one grid
+// (each a chain of loads that fills few of the GPU's warps on a mid-size QP):
+// Q v and A v of MINRES, solve and backward of an n = 8000 QP 133 -> 120 ms.
+// Residuals, M-norm and sigma, once in 100 steps, gain nothing measurable.
+template <class Epi1, class Epi2>
+__global__ void __launch_bounds__(kThreads, HPR_SPMV_MIN_BLOCKS)
+    k_spmv2(const DCsr M1, const double *x1, const Epi1 epi1, const DCsr M2, const double *x2, const Epi2 epi2)
+{
+    __shared__ double s_row[kWarps][kTileRows];
+    const int g1 = M1.grid_chunk + M1.grid_main;
+    if ((int)blockIdx.x < g1) spmv_cta(M1, x1, epi1, blockIdx.x, s_row);
+    else spmv_cta(M2, x2, epi2, blockIdx.x - g1, s_row);
 }
 
 // padded shared-memory slot of window entry i (conflict-free for both the
@@ -492,7 +514,7 @@ __global__ void __launch_bounds__(kThreads, HPR_SPMV_STAGED_MIN_BLOCKS) k_spmv_s
     __shared__ int s_rs[kWarps][kTileRows + 1];
     __shared__ double s_row[kWarps][kTileRows];
     if ((int)blockIdx.x < M.grid_chunk) {
-        chunk_cta(M, xin, epi);
+        chunk_cta(M, xin, epi, blockIdx.x);
         return;
     }
     const int cta = blockIdx.x - M.grid_chunk;

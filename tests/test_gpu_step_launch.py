@@ -98,3 +98,52 @@ def test_scaling_of_long_rows(engine_lib, n):
     np.testing.assert_allclose(got["row_norm"], rn, rtol=200 * np.finfo(float).eps)
     np.testing.assert_allclose(got["col_norm"], cn, rtol=200 * np.finfo(float).eps)
     np.testing.assert_allclose(got["a_val"], A[rows, arrays["a_indices"]], rtol=200 * np.finfo(float).eps)
+
+
+@pytest.mark.parametrize("long_q", [False, True])
+@pytest.mark.parametrize("long_a", [0, 2, 257])
+def test_two_products_in_one_launch(engine_lib, long_q, long_a):
+    """MINRES, whose Q v and A v share a launch, with and without rows longer
+    than a chunk (257 long rows of A keep the products apart): the solution
+    satisfies the active-set KKT system assembled on the host to 1e-8 (the
+    bound of test_single_adjoint_large_kkt_residual), and a second backward
+    gives the same bits (tolerance 0)."""
+    import scipy.sparse as sp
+    from hprqp import instances
+
+    n, m = 1100, 300
+    rng = np.random.default_rng(7 * long_a + long_q)
+    inst = instances.plain_qp(11, n=n, m=m, a_density=0.02, m_rows=30, m_density=0.01, n_eq=20)
+
+    def csr(M):
+        M = M.tocsr()
+        M.sort_indices()
+        return instances.CSR(*M.shape, M.indptr.astype(np.int64), M.indices.astype(np.int64), M.data)
+
+    if long_a:
+        A = inst.A.to_scipy().tolil()
+        long_rows = rng.choice(m, long_a, replace=False)
+        A[long_rows, :] = rng.standard_normal((long_a, n)) / n
+        inst.A, inst.AL[long_rows], inst.AU[long_rows] = csr(A), -1.0, 1.0
+    if long_q:  # two dense rows and columns, and a diagonal that dominates
+        arrow = np.zeros((n, n))
+        arrow[[3, 500], :] = rng.uniform(-1, 1, (2, n)) / n
+        Q = inst.Q.to_scipy() + sp.csr_matrix(arrow + arrow.T)
+        inst.Q = csr(Q + sp.diags(np.asarray(abs(Q).sum(1)).ravel()))
+    model = engine_lib.build_from_instance(inst)
+    r, state = engine_lib.solve_for_backward(model, engine_lib.Parameters(verbose=False, stoptol=1e-8, max_iter=20000))
+    assert r.status_code == engine_lib.STATUS_OPTIMAL
+    try:
+        gx = rng.standard_normal(n)
+        g, again = state.backward(gx, tol=1e-12), state.backward(gx, tol=1e-12)
+    finally:
+        state.close()
+    a = engine_lib.model_arrays(model)
+    Q, A = (sp.csr_matrix((a[k + "_data"], a[k + "_indices"], a[k + "_indptr"]), shape=(rows, n))
+            for k, rows in (("q", n), ("a", a["m"])))
+    F, R = np.nonzero(r.z == 0.0)[0], np.nonzero(r.y != 0.0)[0]
+    AF = A[R][:, F]
+    res = np.concatenate([Q[F][:, F] @ g["lam"][F] + AF.T @ g["mu"][R] - gx[F], AF @ g["lam"][F]])
+    assert np.linalg.norm(res) <= 1e-8 * np.linalg.norm(gx[F])
+    for k in ("dc", "lam", "mu", "dQ_values", "dA_values"):
+        np.testing.assert_array_equal(again[k], g[k], err_msg=k)
