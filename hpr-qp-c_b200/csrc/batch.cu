@@ -503,10 +503,10 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
             V.dQw[i] = V.QATdy[i] = V.dx[i] = V.dw[i] = V.z_bar[i] = V.tempv[i] = 0.0;
             V.last_Qw[i] = V.last_ATy[i] = 0.0;
             if (S.q_is_diag) {
-                const double inv = 1.0 / (1.0 + S.sigma * V.diag_Q[i]);
+                const double inv = diag_inverse(S.sigma, V.diag_Q[i]);
                 V.fact2[i] = inv;
                 V.fact[i] = S.sigma * inv;
-                V.fact1[i] = S.sigma * V.diag_Q[i] * inv;
+                V.fact1[i] = diag_fact1(S.sigma, V.diag_Q[i], inv);
                 V.fact_M[i] = S.sigma * S.sigma * inv;
             }
         }
@@ -601,7 +601,7 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
                     const double z_raw = xi + sigma * (-V.Qw[i] + aty - V.c[i]);
                     const double xb = clampd(z_raw, V.l[i], V.u[i]);
                     const double xh = 2.0 * xb - xi;
-                    const double wb = diag ? V.fact1[i] * wi + V.fact2[i] * xh : f1s * wi + f2s * xh;
+                    const double wb = diag ? w_bar_diag(V.fact1[i], wi, V.fact2[i], xh) : f1s * wi + f2s * xh;
                     if (full) {
                         V.x_bar[i] = xb;
                         V.z_bar[i] = (xb - z_raw) / sigma;
@@ -638,7 +638,7 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
                         V.dx[i] = xb - xi;
                     }
                     V.x[i] = h2 * xh + h1 * V.last_x[i];
-                    V.w_bar[i] = diag ? V.fact1[i] * wi + V.fact2[i] * xh : f1s * wi + f2s * xh;
+                    V.w_bar[i] = diag ? w_bar_diag(V.fact1[i], wi, V.fact2[i], xh) : f1s * wi + f2s * xh;
                 });
                 __syncthreads();
                 if (m > 0) {
@@ -864,10 +864,10 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
             if (S.q_is_diag && fabs(S.sigma - S.scal[0]) > 1e-15) {
                 const double sg = S.sigma;
                 for (int i = tid; i < n; i += kBT) {
-                    const double inv = 1.0 / (1.0 + sg * V.diag_Q[i]);
+                    const double inv = diag_inverse(sg, V.diag_Q[i]);
                     V.fact2[i] = inv;
                     V.fact[i] = sg * inv;
-                    V.fact1[i] = sg * V.diag_Q[i] * inv;
+                    V.fact1[i] = diag_fact1(sg, V.diag_Q[i], inv);
                     V.fact_M[i] = sg * sg * inv;
                 }
                 __syncthreads();

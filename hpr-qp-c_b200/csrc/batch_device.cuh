@@ -121,6 +121,21 @@ __device__ __forceinline__ double clampd(double v, double lo, double hi)
     return v < lo ? lo : (v > hi ? hi : v);
 }
 
+// The factors of a diagonal Q and w_bar, rounded one way wherever they are
+// compiled: an instance may start in k_batch_solve and go on in
+// k_cluster_solve, at a moment that depends on the others, and must not show
+// where it did.  (Left to the compiler, sigma d is fused into 1 + sigma d in
+// one kernel and shared with fact1 in the other.)
+__device__ __forceinline__ double diag_inverse(double sigma, double d) { return 1.0 / fma(sigma, d, 1.0); }
+__device__ __forceinline__ double diag_fact1(double sigma, double d, double inv)
+{
+    return __dmul_rn(__dmul_rn(sigma, d), inv);
+}
+__device__ __forceinline__ double w_bar_diag(double f1, double w, double f2, double x_hat)
+{
+    return fma(f1, w, __dmul_rn(f2, x_hat));
+}
+
 // CTA-shared control state of the instance being solved
 struct CtaState {
     double sigma, lA, lQ;

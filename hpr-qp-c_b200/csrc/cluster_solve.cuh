@@ -786,10 +786,10 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
         auto diag_factors = [&]() {
             const double sg = S.sigma;
             for (int i = tid; i < nl; i += NT) {
-                const double dq = V.diag_Q[nr0 + i], inv = 1.0 / (1.0 + sg * dq);
+                const double dq = V.diag_Q[nr0 + i], inv = diag_inverse(sg, dq);
                 V.fact2[nr0 + i] = inv;
                 V.fact[nr0 + i] = sg * inv;
-                V.fact1[nr0 + i] = sg * dq * inv;
+                V.fact1[nr0 + i] = diag_fact1(sg, dq, inv);
                 V.fact_M[nr0 + i] = sg * sg * inv;
             }
         };
@@ -935,7 +935,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
                     const double z_raw = xi + sigma * (-own[kClNOwn * i + kQw] + aty - own[kClNOwn * i + kC]);
                     const double xb = clampd(z_raw, own[kClNOwn * i + kL], own[kClNOwn * i + kU]);
                     const double xh = 2.0 * xb - xi;
-                    const double wb = diag ? V.fact1[nr0 + i] * wi + V.fact2[nr0 + i] * xh : f1s * wi + f2s * xh;
+                    const double wb = diag ? w_bar_diag(V.fact1[nr0 + i], wi, V.fact2[nr0 + i], xh) : f1s * wi + f2s * xh;
                     push(G2 + gi, wb, kBarWb);
                     if (full) {
                         V.x_bar[gi] = xb;
@@ -965,7 +965,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
                     const double z_raw = xi + sigma * (-qw + own[kClNOwn * i + kAty] - own[kClNOwn * i + kC]);
                     const double xb = clampd(z_raw, own[kClNOwn * i + kL], own[kClNOwn * i + kU]);
                     const double xh = 2.0 * xb - xi;
-                    const double wb = diag ? V.fact1[nr0 + i] * wi + V.fact2[nr0 + i] * xh : f1s * wi + f2s * xh;
+                    const double wb = diag ? w_bar_diag(V.fact1[nr0 + i], wi, V.fact2[nr0 + i], xh) : f1s * wi + f2s * xh;
                     push(G2 + gi, wb, kBarWb);
                     own[kClNOwn * i + kQw] = qw;
                     own[kClNOwn * i + kXh] = xh;

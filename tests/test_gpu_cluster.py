@@ -89,3 +89,34 @@ def test_handed_over_instances(engine_lib, count):
         s = alone.results()
         assert s.iter[0] == r.iter[k] and s.status[0] == r.status[k]
         np.testing.assert_array_equal(s.x, xs[k])
+
+
+@pytest.mark.parametrize("max_iter", [1, 230])
+@pytest.mark.parametrize("kind", ["boxed", "free"])
+@pytest.mark.parametrize("count", [200, 308])
+def test_diagonal_q_equals_one_cta(engine_lib, count, kind, max_iter):
+    """Instances whose Q is diagonal: on the one-CTA kernel (the batch of 308
+    holds shapes that k_cluster_solve takes and shapes that it does not) and
+    on clusters the same bits, so a hand-over does not show."""
+    from hprqp import instances
+    from hprqp.batch import Batch, pack
+
+    insts = []
+    for i, inst in enumerate(_instances(kind)):
+        n = inst.n
+        d = np.random.default_rng(i).uniform(0.1, 2.0, n)
+        inst.Q = instances.CSR(n, n, np.arange(n + 1), np.arange(n), d)
+        insts.append(inst)
+    kw = dict(stoptol=1e-30, max_iter=max_iter)
+    many = Batch(pack((insts * 28)[:count]))
+    many.solve(**kw)
+    ref = many.results()
+    many.solve(**kw)
+    again = many.results()
+    few = Batch(pack(insts))
+    few.solve(**kw)
+    got = few.results()
+    for f, size in (("x", few.n), ("w", few.n), ("z", few.n), ("y", few.m)):
+        np.testing.assert_array_equal(getattr(again, f), getattr(ref, f), err_msg=f)
+        if count > 296:  # (up to 296 instances the sums are taken in another order)
+            np.testing.assert_array_equal(getattr(got, f), getattr(ref, f)[:size], err_msg=f)
