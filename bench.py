@@ -248,7 +248,7 @@ def objective_agreement(ours_status, ours_obj, ref_solved):
 def plain_call_stats(seconds, product_nnz, one_cta_limit: int = 200000):
     """Per-call summary of the plain loop: median and slowest call, and the
     slowest call's instance and route (solve_gpu runs a model without cones
-    on one CTA of the batch kernel when 2 nnz(Q) + 2 nnz(A) <= the limit,
+    as a batch of one when 2 nnz(Q) + 2 nnz(A) <= the limit,
     else through the host-driven loop)."""
     ms = [1e3 * float(t) for t in seconds]
     if not ms:
@@ -730,11 +730,14 @@ def main():
                     "optimal": e2e_ok},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": algo_bytes * BATCH_DRAM_PER_ALGO_BYTE,
-                         "traffic_source": "ncu DRAM bytes of a 300-QP solve of this workload (same kernel "
-                                           "shapes), scaled by algorithmic bytes (instance-iterations)",
-                         "kernel": "k_batch_solve (one solve: a 640-thread launch for the instances of "
-                                   "n, m <= 640 and a 1024-thread launch for the rest, concurrent; "
-                                   "achieved over their span)",
+                         "traffic_source": "estimate: ncu DRAM bytes of a 300-QP solve of this workload with every "
+                                           "instance in k_batch_solve (the small ones now run in "
+                                           "k_cluster_solve's one-CTA form), scaled by algorithmic bytes "
+                                           "(instance-iterations)",
+                         "kernel": "k_batch_solve and k_cluster_solve (one solve: a one-CTA launch for "
+                                   "the instances of n, m <= 640 and a 1024-thread launch for the "
+                                   "rest, concurrent, the last ones handed to clusters; achieved over "
+                                   "their span)",
                          "algorithmic_bytes_per_launch": algo_bytes, "peak_kind": peak_kind},
             "solved_optimal": int(np.sum(res.status == 6)), "mean_iters": float(iters.mean())}
 
@@ -764,7 +767,7 @@ def main():
         finally:
             hprqp.set_single_cta_max_work(old_route)
         line["plain"] = {"value": plain_rate, "unit": "solves/s", "sample": f"{len(models)} instances of the batch",
-                         "route": "one CTA of the batch kernel per solve_gpu call (small models)",
+                         "route": "one thread-block cluster per solve_gpu call (small models)",
                          "host_loop": host_loop_rate, "calls": calls}
         line["batched_over_plain"] = value / world / plain_rate
         line["batched_over_plain_host_loop"] = value / world / host_loop_rate

@@ -23,6 +23,11 @@
 // is structural, so an instance sums in the same order in every solve; every
 // reduction is folded in a fixed order, so each instance's result is
 // independent of which CTA solved it.
+//
+// Where there are fewer instances than SMs -- a small batch, or the last ones
+// of a large one, which k_batch_solve then hands over -- an instance runs on a
+// thread-block cluster (k_cluster_solve, cluster_solve.cuh), with the same
+// results.
 #include "engine.h"
 #include "hprqp_batch.h"
 #include "hprqp.h"

@@ -91,7 +91,7 @@ HPRQPStatus hprqp_b200_power_lambda_noalloc(int device, size_t m, size_t n, cons
 /* Routing of solve_gpu (an addition: the reference runs every model through
  * its host-driven loop, src/shared/solver_backend.c:432-513).  A model
  * without cones whose products per iteration touch at most max_work
- * nonzeros (2 nnz(Q) + 2 nnz(A)) is solved in one CTA of the batch kernel
+ * nonzeros (2 nnz(Q) + 2 nnz(A)) is solved as a batch of one on the device
  * -- same method, same results up to rounding, one launch instead of host
  * round trips per iteration -- unless it is solved for the adjoint
  * (hprqp_solve_for_backward).  max_work = 0 sends every model through the
