@@ -42,7 +42,7 @@ sys.path.insert(0, str(ROOT / "hpr-qp-c_b200" / "python"))
 sys.path.insert(0, str(ROOT / "oracle"))
 
 # DRAM bytes moved per algorithmic byte by k_batch_solve: ncu on a 300-QP
-# solve of this workload in the bench's kernel shapes (a 640-thread launch
+# solve of this workload, every instance in k_batch_solve (a 640-thread launch
 # for its 85 instances of n, m <= 640, a 1024-thread launch for the rest, one
 # instance per SM at a time, no shared-memory pool) read+wrote 0.009 +
 # 394.424 GB (dram__bytes_read.sum + dram__bytes_write.sum of both launches)
