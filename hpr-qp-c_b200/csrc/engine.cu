@@ -636,14 +636,14 @@ struct EpiRestart : EpiBase<0> {
             S.last_Qw[i] = q;
         }
     }
-    __device__ void extra(Acc<0> &, int cta, int) const
+    __device__ void extra(Acc<0> &, int cta, int ctas) const
     {
-        for (int i = blockIdx.x * kThreads + threadIdx.x; i < S.m; i += gridDim.x * kThreads) {
+        for (int i = cta * kThreads + threadIdx.x; i < S.m; i += ctas * kThreads) {
             const double yb = S.y_bar[i];
             S.y[i] = yb;
             S.last_y[i] = yb;
         }
-        if (blockIdx.x == 0 && threadIdx.x == 0) {
+        if (cta == 0 && threadIdx.x == 0) {
             S.ctl->inner = 0;
             S.ctl->inner_next = 0;
         }

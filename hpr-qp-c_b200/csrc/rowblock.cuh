@@ -272,6 +272,8 @@ __device__ __forceinline__ void tile_rowsums(const DCsr &M, const double *x, int
 //   static constexpr int NRED;  __host__ __device__ void ops(int*) const;
 //   __device__ void init(Acc&) const; row(int i, double y_i, Acc&) const;
 //   __device__ void extra(Acc&, int cta, int ctas) const;  // once per CTA, tiles only
+//     (cta of ctas: its place among them; blockIdx counts the chunk CTAs, which
+//     come first in the grid and never call it)
 //   double *partials;                         // [npart * NRED]
 // the long rows' epilogue: adds the chunk partials of row i in order
 template <class Epi>
