@@ -1264,6 +1264,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
         };
         step_constants();
         if (!resume) {
+            save_w_bar();
             residuals(0, false);
             if (tid == 0) {
                 S.got4 = S.got6 = 0;
@@ -1322,7 +1323,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
                     S.print_yes = print_yes;
                 }
                 __syncthreads();
-                save_w_bar();
+                if (iter > 0) save_w_bar();  // (iteration 0's residuals have taken w_bar's buffer)
                 PHASE_ADD(3);
                 if (S.do_res) residuals(iter, on_grid && !noC);
                 PHASE_ADD(4);
