@@ -349,7 +349,7 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
                 B.restarts[k] = 0;
                 B.sigma_out[k] = 0.0;
                 B.seconds_out[k] = 0.0;
-                atomicAdd(B.finished, 1ull);
+                count_finished(B, I);
             }
             __syncthreads();
             continue;
@@ -1096,7 +1096,7 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
             B.sigma_out[k] = S.sigma;
             B.seconds_out[k] = 1e-9 * (double)(globaltimer_ns() - inst_t0);
             if (B.loop_seconds_out) B.loop_seconds_out[k] = 1e-9 * (double)(globaltimer_ns() - loop_t0);
-            atomicAdd(B.finished, 1ull);
+            count_finished(B, I);
         }
         __syncthreads();
     }
@@ -1294,6 +1294,11 @@ __global__ void k_batch_clock(unsigned long long *t)
     *t = globaltimer_ns();
 }
 
+__global__ void k_batch_hold(unsigned long long *hold, long long change)
+{
+    atomicAdd(hold, (unsigned long long)change);
+}
+
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
@@ -1343,8 +1348,8 @@ struct Group {
     size_t first, count;
 };
 constexpr int kMaxGroups = 12;                    // 2 shapes x {0, 1, 2, 4, 8, 16}
-constexpr int kCounters = kMaxGroups + 2;         // one queue per launch, finished, handed over
-constexpr int kFinished = kMaxGroups, kHandedOver = kMaxGroups + 1;
+constexpr int kCounters = kMaxGroups + 3;         // one queue per launch, finished, handed over, hold
+constexpr int kFinished = kMaxGroups, kHandedOver = kMaxGroups + 1, kHold = kMaxGroups + 2;
 }  // namespace hpr
 
 struct HPRQPBatch {
@@ -1359,9 +1364,10 @@ struct HPRQPBatch {
     // instances handed from one phase to the next (allocated by the first
     // solve with more than one phase): records of two phases, work order
     // a part of a call that solves k_total instances counts the finished ones
-    // of all parts in one place
+    // of all parts, and what holds a hand-over up (BatchArgs::hold), in one place
     int k_total = 0;
-    unsigned long long *finished = nullptr;
+    unsigned long long *finished = nullptr, *hold = nullptr;
+    int hold_change = 0;  // added to it by the solve's first launch
     std::vector<int> order, phase_ids;  // instances of the first and of the current phase's entries
     hpr::BResume *resume[2] = {nullptr, nullptr};
     int *resume_order = nullptr;
@@ -1982,6 +1988,7 @@ static HPRQPStatus batch_create_impl(size_t K, const size_t *var_offsets, const 
         I.obj_constant = M.obj_constant;
         I.movable = 0;
         for (int C = 16; C >= 1; C >>= 1) I.movable |= cluster_fits(b, k, C);
+        b->hold_change += !I.movable;
         // every instance's entries start on a 4-entry (16-byte) boundary, so
         // cta_spmv can read aligned quads of indices and values
         qnz += (M.Q.nnz + 3) & ~size_t(3);
@@ -2279,6 +2286,11 @@ static HPRQPStatus phase_launch(HPRQPBatch *b, SolveLaunch &L, const int *order,
     // the queues of this phase; the count of finished instances goes on
     B_CK(cudaMemsetAsync(G.counter, 0, (in ? kMaxGroups : kCounters) * sizeof(*G.counter), b->stream));
     if (in) B_CK(cudaMemsetAsync(G.counter + kHandedOver, 0, sizeof(*G.counter), b->stream));
+    unsigned long long *const hold = b->hold ? b->hold : G.counter + kHold;
+    if (!in && b->hold_change) {
+        k_batch_hold<<<1, 1, 0, b->stream>>>(hold, b->hold_change);
+        count_launch();
+    }
     // the next phase: with a quarter of the running instances left, each of
     // them can have four times the SMs (400 QPs of the batch recipe, limit
     // 20,000 iterations: 418 ms without, 296 ms with the phases 37, 9 and 2
@@ -2320,6 +2332,7 @@ static HPRQPStatus phase_launch(HPRQPBatch *b, SolveLaunch &L, const int *order,
         A.K_total = b->k_total ? b->k_total : (int)b->K;
         A.yield_at = L.yield_at;
         A.finished = b->finished ? b->finished : G.counter + kFinished;
+        A.hold = hold;
         A.resume_count = G.counter + kHandedOver;
         A.resume_out = b->resume[L.phase & 1];
         A.resume_in = in;
@@ -2919,6 +2932,8 @@ static HPRQPStatus solve_batch_in_two(size_t K, const size_t *var_offsets, const
             // instances are handed over when few of both parts are left
             b[part]->k_total = (int)K;
             b[part]->finished = b[0]->args.counter + kFinished;
+            b[part]->hold = b[0]->args.counter + kHold;
+            b[part]->hold_change += part == 0 ? 1 : -1;  // the second part is still to come
             st = batch_launch(b[part], params, L[part]);
         }
         if (st == HPRQP_STATUS_OK) ++launched;

@@ -72,9 +72,13 @@ struct BatchArgs {
     // K_total instances are unfinished and this launch's queue is empty, the
     // running instances are saved (state in their workspace slots, control
     // state in resume_out) and their CTAs end, so that a next launch can give
-    // each of them more SMs.  resume_in: the instances this launch goes on
-    // with (its order then lists records).
+    // each of them more SMs.  The next launch waits for all of a phase's, so
+    // nothing is handed over while *hold > 0: it counts the unfinished
+    // instances that no cluster takes and the parts of the call that are not
+    // launched yet.  resume_in: the instances this launch goes on with (its
+    // order then lists records).
     int K_total, yield_at;
+    unsigned long long *hold;
     int slot0;                         // workspace slot of this launch's CTA (cluster) 0
     double *ws_all;                    // workspace slot 0
     unsigned long long *finished;      // instances finished so far, over all launches
@@ -171,7 +175,15 @@ static __device__ __forceinline__ bool yield_now(const BatchArgs &B, const BInst
     if (B.yield_at <= 0 || !I.movable) return false;
     const unsigned long long taken = *(volatile unsigned long long *)B.counter;
     if ((taken & 0xffffffffull) + (taken >> 32) < (unsigned long long)B.K) return false;
-    return (long long)B.K_total - (long long)*(volatile unsigned long long *)B.finished <= (long long)B.yield_at;
+    return (long long)B.K_total - (long long)*(volatile unsigned long long *)B.finished <= (long long)B.yield_at &&
+           *(volatile unsigned long long *)B.hold == 0;
+}
+
+// instance I has ended
+static __device__ __forceinline__ void count_finished(const BatchArgs &B, const BInst &I)
+{
+    atomicAdd(B.finished, 1ull);
+    if (!I.movable) atomicAdd(B.hold, ~0ull);
 }
 
 struct Vecs {

@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
                     B.restarts[k] = 0;
                     B.sigma_out[k] = 0.0;
                     B.seconds_out[k] = 0.0;
-                    atomicAdd(B.finished, 1ull);
+                    count_finished(B, I);
                 }
             }
             continue;
@@ -1463,7 +1463,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
             B.sigma_out[k] = S.sigma;
             B.seconds_out[k] = 1e-9 * (double)(globaltimer_ns() - inst_t0);
             if (B.loop_seconds_out) B.loop_seconds_out[k] = 1e-9 * (double)(globaltimer_ns() - loop_t0);
-            atomicAdd(B.finished, 1ull);
+            count_finished(B, I);
         }
         sync();
         if (MULTI && s_dead) break;

@@ -30,3 +30,21 @@ def test_warm_start_without_a_step(engine_lib, n, count):
     assert np.all(r.iter == 0)
     for got, want in ((r.x, x), (r.w, w), (r.y, y)):
         np.testing.assert_allclose(got, want, rtol=4 * np.finfo(float).eps, atol=0)
+
+
+def test_movable_instances_do_not_wait_for_others(engine_lib):
+    """Seven small QPs beside one that no cluster takes (n > 8190) and that
+    runs into the time limit: the small ones, 60,000 steps of a few
+    microseconds, end by their iteration limit long before it."""
+    from hprqp.batch import Batch, pack
+
+    small = [instances.plain_qp(60 + i, n=n, m=n // 2, a_density=0.1, m_rows=10, m_density=0.05, n_eq=5)
+             for i, n in enumerate([40] * 6 + [500])]
+    large = instances.plain_qp(70, n=8200, m=2000, a_density=0.002, m_rows=1640, m_density=0.002, n_eq=500)
+    b = Batch(pack(small + [large]))
+    b.solve(stoptol=1e-30, max_iter=60000, time_limit=2.0)
+    r = b.results(vectors=False)
+    b.close()
+    assert r.status[-1] == 5 and 0 < r.iter[-1] < 60000, (r.status[-1], r.iter[-1])
+    np.testing.assert_array_equal(r.status[:-1], 4)
+    np.testing.assert_array_equal(r.iter[:-1], 60000)
