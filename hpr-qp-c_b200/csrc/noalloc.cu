@@ -34,44 +34,11 @@
 #include "pool.h"
 #include "rowblock.cuh"
 
-#include <cuda.h>
 #include <cuda_runtime.h>
 
 #include <cmath>
 #include <cstdio>
 #include <mutex>
-
-namespace hpr {
-
-// Identity of the current context (cuCtxGetId, reached through the runtime's
-// driver entry points so the library links only cudart); false when the
-// driver does not offer it.
-bool current_context_id(unsigned long long *id)
-{
-    using GetCurrentFn = CUresult (*)(CUcontext *);
-    using GetIdFn = CUresult (*)(CUcontext, unsigned long long *);
-    static GetCurrentFn get_current = nullptr;
-    static GetIdFn get_id = nullptr;
-    static bool looked_up = false;
-    if (!looked_up) {
-        void *f0 = nullptr, *f1 = nullptr;
-        cudaDriverEntryPointQueryResult q0, q1;
-        if (cudaGetDriverEntryPoint("cuCtxGetCurrent", &f0, cudaEnableDefault, &q0) == cudaSuccess &&
-            q0 == cudaDriverEntryPointSuccess && cudaGetDriverEntryPoint("cuCtxGetId", &f1, cudaEnableDefault, &q1) ==
-                                                     cudaSuccess && q1 == cudaDriverEntryPointSuccess) {
-            get_current = (GetCurrentFn)f0;
-            get_id = (GetIdFn)f1;
-        }
-        cudaGetLastError();  // a missing entry point is not an error of this call
-        looked_up = true;
-    }
-    if (!get_current || !get_id) return false;
-    CUcontext ctx = nullptr;
-    if (get_current(&ctx) != CUDA_SUCCESS || ctx == nullptr) return false;
-    return get_id(ctx, id) == CUDA_SUCCESS;
-}
-
-}  // namespace hpr
 
 namespace hpr_noalloc {
 

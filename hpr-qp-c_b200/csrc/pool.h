@@ -34,7 +34,7 @@ void pool_stream_return(cudaStream_t s);
 void *pool_pinned(void **dev);
 void pool_pinned_return(void *host);
 
-// identity of the current context (noalloc.cu)
+// identity of the current context; false when there is none (context_id.cpp)
 bool current_context_id(unsigned long long *id);
 
 }  // namespace hpr
