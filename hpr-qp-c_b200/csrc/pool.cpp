@@ -130,8 +130,8 @@ void pool_free(void *p)
             return;
         }
         cudaFree(p);
-    } else if (keyed && b.key.device != k.device) {
-        cudaFree(p);  // another device's block: freed by address
+    } else if (!keyed || b.key.device != k.device) {
+        cudaFree(p);  // another device's block, or no telling whose: freed by address
     }
     // (a block of a context that is gone went with it)
 }

@@ -8,11 +8,15 @@
 #include <atomic>
 #include <chrono>
 #include <cstdio>
+#include <cstdlib>
 #include <cstring>
+#include <set>
 #include <thread>
 #include <vector>
 
 static std::atomic<int> lookups{0};
+static bool ids = true;           // the driver answers
+static std::set<void *> held;     // device blocks that are allocated
 
 static CUresult get_current(CUcontext *c)
 {
@@ -22,7 +26,7 @@ static CUresult get_current(CUcontext *c)
 static CUresult get_id(CUcontext, unsigned long long *id)
 {
     *id = 7;
-    return CUDA_SUCCESS;
+    return ids ? CUDA_SUCCESS : CUDA_ERROR_UNKNOWN;
 }
 
 extern "C" {
@@ -35,6 +39,46 @@ cudaError_t cudaGetDriverEntryPoint(const char *name, void **f, unsigned long lo
     return cudaSuccess;
 }
 cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaGetDevice(int *d)
+{
+    *d = 0;
+    return cudaSuccess;
+}
+cudaError_t cudaMalloc(void **p, size_t bytes)
+{
+    held.insert(*p = malloc(bytes));
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void *p)
+{
+    if (p && held.erase(p)) free(p);
+    return cudaSuccess;
+}
+cudaError_t cudaHostAlloc(void **p, size_t bytes, unsigned)
+{
+    *p = malloc(bytes);
+    return cudaSuccess;
+}
+cudaError_t cudaHostGetDevicePointer(void **d, void *h, unsigned)
+{
+    *d = h;
+    return cudaSuccess;
+}
+cudaError_t cudaFreeHost(void *p)
+{
+    free(p);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned)
+{
+    *s = (cudaStream_t)malloc(1);
+    return cudaSuccess;
+}
+cudaError_t cudaStreamDestroy(cudaStream_t s)
+{
+    free(s);
+    return cudaSuccess;
+}
 }
 
 // eight threads that ask for the first time at once: one lookup of each of the
@@ -55,8 +99,20 @@ static int first_use()
     return lookups == 2 && answers == 8 ? 0 : 1;
 }
 
+// a block that the pool has on record, returned while the context's identity
+// cannot be read: given back to the device, not forgotten
+static int unknown_context()
+{
+    void *p = hpr::pool_alloc(1000);
+    ids = false;
+    hpr::pool_free(p);
+    printf("%zu blocks still allocated\n", held.size());
+    return held.empty() ? 0 : 1;
+}
+
 int main(int argc, char **argv)
 {
     if (argc == 2 && !strcmp(argv[1], "first_use")) return first_use();
+    if (argc == 2 && !strcmp(argv[1], "unknown_context")) return unknown_context();
     return 2;
 }

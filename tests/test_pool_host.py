@@ -23,11 +23,12 @@ def probe(tmp_path_factory):
     env = {k: v for k, v in os.environ.items() if k != "LD_PRELOAD"}
     csrc = ROOT / "hpr-qp-c_b200" / "csrc"
     subprocess.run([cxx, "-std=c++17", "-O1", "-pthread", f"-I{csrc}", f"-I{cuda}/include", "-o", str(exe),
-                    str(ROOT / "tests" / "native" / "pool_probe.cpp"), str(csrc / "context_id.cpp")],
+                    str(ROOT / "tests" / "native" / "pool_probe.cpp"), str(csrc / "context_id.cpp"), str(csrc / "pool.cpp")],
                    check=True, env=env)
     return lambda case: subprocess.run([str(exe), case], capture_output=True, text=True, timeout=60, env=env)
 
 
-def test_first_use_from_several_threads(probe):
-    r = probe("first_use")
+@pytest.mark.parametrize("case", ["first_use", "unknown_context"])
+def test_probe(probe, case):
+    r = probe(case)
     assert r.returncode == 0, r.stdout + r.stderr
