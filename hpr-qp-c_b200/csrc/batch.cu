@@ -3139,3 +3139,14 @@ extern "C" size_t hprqp_b200_set_single_cta_max_work(size_t max_work)
     hpr::g_single_cta_max_work = max_work;
     return old;
 }
+
+extern "C" HPRQPStatus hprqp_b200_release_memory(int device)
+{
+    int ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess) {
+        cudaGetLastError();
+        ndev = 0;
+    }
+    if (device < 0 || device >= ndev) return HPRQP_STATUS_INVALID_ARGUMENT;
+    return hpr::pool_release(device) ? HPRQP_STATUS_OK : HPRQP_STATUS_NOT_IMPLEMENTED;
+}

@@ -227,4 +227,26 @@ void pool_pinned_return(void *host)
     cudaFreeHost(host);
 }
 
+bool pool_release(int device)
+{
+    {
+        std::lock_guard<std::mutex> lock(mu);
+        if (!caches().count(device)) return true;  // (nothing kept: leaves a device without a context alone)
+    }
+    int current = -1;
+    if (cudaGetDevice(&current) != cudaSuccess || cudaSetDevice(device) != cudaSuccess) return false;
+    Key k;
+    const bool keyed = here(k);
+    if (keyed) {
+        std::lock_guard<std::mutex> lock(mu);
+        Cache &c = cache_of(k);
+        for (auto &b : c.blocks) cudaFree(b.second);
+        for (auto &s : c.streams) cudaStreamDestroy(s);
+        for (auto &p : c.pinned) cudaFreeHost(p.host);
+        caches().erase(device);
+    }
+    cudaSetDevice(current);
+    return keyed;
+}
+
 }  // namespace hpr

@@ -6,7 +6,7 @@
 // when a solve ends and the next one on the same device takes them.  The pool
 // is bounded (kPoolBytes of device memory a device, kPoolObjects of the
 // rest); what does not fit is freed, and all of it is freed when an
-// allocation fails.  All functions work on the current device, may be called
+// allocation fails or the caller asks (hprqp_b200_release_memory).  All functions work on the current device, may be called
 // from any thread, and drop what belongs to a context that no longer exists.
 #pragma once
 
@@ -33,6 +33,10 @@ void pool_stream_return(cudaStream_t s);
 // device's)
 void *pool_pinned(void **dev);
 void pool_pinned_return(void *host);
+
+// free what the pool keeps on a device (objects in use are not the pool's);
+// false when the device cannot be reached
+bool pool_release(int device);
 
 // identity of the current context; false when there is none (context_id.cpp)
 bool current_context_id(unsigned long long *id);

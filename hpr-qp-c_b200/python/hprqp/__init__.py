@@ -163,6 +163,7 @@ class _Library:
         lib.hprqp_b200_launch_count.restype = ctypes.c_uint64
         lib.hprqp_b200_set_single_cta_max_work.argtypes = [ctypes.c_size_t]
         lib.hprqp_b200_set_single_cta_max_work.restype = ctypes.c_size_t
+        lib.hprqp_b200_release_memory.argtypes = [ctypes.c_int]
         lib.params_set_defaults.argtypes = [ctypes.POINTER(_ParamsStruct)]
         lib.params_set_defaults.restype = None
 
@@ -194,6 +195,12 @@ def set_single_cta_max_work(max_work: int) -> int:
     one CTA of the batch kernel; 0 sends every model through the host-driven
     loop.  Returns the previous value (hprqp_b200_set_single_cta_max_work)."""
     return int(_lib().hprqp_b200_set_single_cta_max_work(int(max_work)))
+
+
+def release_memory(device_number: int = 0) -> None:
+    """Free the device memory that closed handles and finished solves have
+    left for the next ones, at most 512 MB (hprqp_b200_release_memory)."""
+    _raise_for_status(_lib().hprqp_b200_release_memory(int(device_number)), "hprqp_b200_release_memory")
 
 
 def _raise_for_status(code: int, context: str) -> int:

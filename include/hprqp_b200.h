@@ -98,6 +98,15 @@ HPRQPStatus hprqp_b200_power_lambda_noalloc(int device, size_t m, size_t n, cons
  * host-driven loop.  Process-wide; returns the previous value. */
 size_t hprqp_b200_set_single_cta_max_work(size_t max_work);
 
+/* Device blocks, streams and a little pinned host memory are kept when a
+ * handle is closed or a solve ends, for the next one: at most 512 MB a device
+ * (what does not fit is freed at once, all of it when an allocation of this
+ * library fails).  This call frees what is kept on a device, for a program
+ * whose other allocators need it; what open handles and running solves hold
+ * is not touched.  Any thread may call it.  HPRQP_STATUS_INVALID_ARGUMENT for
+ * a device that does not exist. */
+HPRQPStatus hprqp_b200_release_memory(int device);
+
 /* Number of engine kernel launches issued by this process so far
  * (graph replays count each captured kernel). */
 uint64_t hprqp_b200_launch_count(void);

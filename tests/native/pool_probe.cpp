@@ -16,7 +16,7 @@
 
 static std::atomic<int> lookups{0};
 static bool ids = true;           // the driver answers
-static std::set<void *> held;     // device blocks that are allocated
+static std::set<void *> held;     // blocks, pinned words and streams that exist
 
 static CUresult get_current(CUcontext *c)
 {
@@ -44,6 +44,7 @@ cudaError_t cudaGetDevice(int *d)
     *d = 0;
     return cudaSuccess;
 }
+cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 cudaError_t cudaMalloc(void **p, size_t bytes)
 {
     held.insert(*p = malloc(bytes));
@@ -56,7 +57,7 @@ cudaError_t cudaFree(void *p)
 }
 cudaError_t cudaHostAlloc(void **p, size_t bytes, unsigned)
 {
-    *p = malloc(bytes);
+    held.insert(*p = malloc(bytes));
     return cudaSuccess;
 }
 cudaError_t cudaHostGetDevicePointer(void **d, void *h, unsigned)
@@ -66,19 +67,10 @@ cudaError_t cudaHostGetDevicePointer(void **d, void *h, unsigned)
 }
 cudaError_t cudaFreeHost(void *p)
 {
-    free(p);
-    return cudaSuccess;
+    return cudaFree(p);
 }
-cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned)
-{
-    *s = (cudaStream_t)malloc(1);
-    return cudaSuccess;
-}
-cudaError_t cudaStreamDestroy(cudaStream_t s)
-{
-    free(s);
-    return cudaSuccess;
-}
+cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, unsigned) { return cudaMalloc((void **)s, 1); }
+cudaError_t cudaStreamDestroy(cudaStream_t s) { return cudaFree(s); }
 }
 
 // eight threads that ask for the first time at once: one lookup of each of the
@@ -110,9 +102,27 @@ static int unknown_context()
     return held.empty() ? 0 : 1;
 }
 
+// what the pool keeps can be had back; what is in use stays
+static int release()
+{
+    void *dev = nullptr, *kept[2] = {hpr::pool_alloc(1000), hpr::pool_alloc(5000)}, *used = hpr::pool_alloc(100000);
+    cudaStream_t s = hpr::pool_stream();
+    void *word = hpr::pool_pinned(&dev);
+    for (void *p : kept) hpr::pool_free(p);
+    hpr::pool_stream_return(s);
+    hpr::pool_pinned_return(word);
+    const size_t before = held.size();
+    const bool ok = hpr::pool_release(0) && hpr::pool_release(1);
+    printf("%zu objects, %zu after the release\n", before, held.size());
+    if (!ok || before != 5 || held.size() != 1 || !held.count(used)) return 1;
+    hpr::pool_free(used);  // kept again
+    return held.size() == 1 && hpr::pool_alloc(100000) == used ? 0 : 1;
+}
+
 int main(int argc, char **argv)
 {
     if (argc == 2 && !strcmp(argv[1], "first_use")) return first_use();
     if (argc == 2 && !strcmp(argv[1], "unknown_context")) return unknown_context();
+    if (argc == 2 && !strcmp(argv[1], "release")) return release();
     return 2;
 }

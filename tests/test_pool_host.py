@@ -28,7 +28,7 @@ def probe(tmp_path_factory):
     return lambda case: subprocess.run([str(exe), case], capture_output=True, text=True, timeout=60, env=env)
 
 
-@pytest.mark.parametrize("case", ["first_use", "unknown_context"])
+@pytest.mark.parametrize("case", ["first_use", "unknown_context", "release"])
 def test_probe(probe, case):
     r = probe(case)
     assert r.returncode == 0, r.stdout + r.stderr
