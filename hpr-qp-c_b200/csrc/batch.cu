@@ -1425,7 +1425,9 @@ static HPRQPStatus balloc(HPRQPBatch *b, T **p, size_t count)
 // Several device arrays carved out of one allocation (256-byte aligned
 // slices): a batch's arrays are created together and freed together, and
 // one cudaMalloc instead of forty keeps small batches (and solve_gpu of a
-// small model) cheap to set up.
+// small model) cheap to set up.  One allocation also means all or none: a
+// failed one leaves no array of a group behind for a later call to take as a
+// sign that the others exist.
 class Carver {
 public:
     template <class T>
@@ -2299,10 +2301,9 @@ static HPRQPStatus phase_launch(HPRQPBatch *b, SolveLaunch &L, const int *order,
     L.yield_at = running >= 8 ? running / 4 : 0;
     if (L.yield_at > 0 && !b->resume[0]) {
         const size_t most = (size_t)std::max(slots, 2 * b->num_sms);
-        HPRQPStatus st;
-        if ((st = balloc(b, &b->resume[0], most)) || (st = balloc(b, &b->resume[1], most)) ||
-            (st = balloc(b, &b->resume_order, most)))
-            return st;
+        Carver cv;
+        cv.add(&b->resume[0], most).add(&b->resume[1], most).add(&b->resume_order, most);
+        if (HPRQPStatus st = cv.commit(b)) return st;
     }
     if (!L.e0) B_CK(cudaEventCreate(&L.e0));
     for (int s = 0; s < ns; ++s)
@@ -2522,11 +2523,11 @@ HPRQPStatus hprqp_batch_set_warm_start(HPRQPBatch *b, const double *x0, const do
         for (size_t i = 0; i < b->total_m_orig; ++i)
             if (!std::isfinite(y0[i])) return HPRQP_STATUS_INVALID_ARGUMENT;
     B_CK(cudaSetDevice(b->device));
-    HPRQPStatus st;
-    if (!b->start_x &&
-        ((st = balloc(b, &b->start_x, N)) || (st = balloc(b, &b->start_w, N)) || (st = balloc(b, &b->start_y, M)) ||
-         (st = balloc(b, &b->start_sigma, b->K))))
-        return st;
+    if (!b->start_x) {
+        Carver cv;
+        cv.add(&b->start_x, N).add(&b->start_w, N).add(&b->start_y, M).add(&b->start_sigma, b->K);
+        if (HPRQPStatus st = cv.commit(b)) return st;
+    }
     // y0 is given on the caller's rows: keep the rows the builder kept
     std::vector<double> hy(std::max<size_t>(M, 1), 0.0);
     if (y0)
@@ -2679,10 +2680,10 @@ HPRQPStatus hprqp_batch_backward(HPRQPBatch *b, const double *grad_x, const doub
     const int grid = std::max(1, std::min((int)K, b->num_sms * std::max(per_sm, 1)));
     const size_t stride = kAdjGlobalN * na + kAdjGlobalM * ma + (lanczos_smem ? 0 : (size_t)kAdjLanczos * (na + ma));
     if (!b->adj_gx) {
-        if ((st = balloc(b, &b->adj_gx, N)) || (st = balloc(b, &b->adj_gy, M)) || (st = balloc(b, &b->adj_lx, N)) ||
-            (st = balloc(b, &b->adj_ly, M)) || (st = balloc(b, &b->adj_rel, K)) || (st = balloc(b, &b->adj_it, K)) ||
-            (st = balloc(b, &b->adj_counter, 1)))
-            return st;
+        Carver cv;
+        cv.add(&b->adj_gx, N).add(&b->adj_gy, M).add(&b->adj_lx, N).add(&b->adj_ly, M);
+        cv.add(&b->adj_rel, K).add(&b->adj_it, K).add(&b->adj_counter, 1);
+        if ((st = cv.commit(b))) return st;
     }
     if (b->adj_ws_count < stride * (size_t)grid) {
         if ((st = balloc(b, &b->adj_ws, stride * (size_t)grid))) return st;
