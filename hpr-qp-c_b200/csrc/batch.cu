@@ -1586,12 +1586,6 @@ static bool mid_cta_instance(const HPRQPModel &M)
 
 namespace hpr {
 
-// dynamic shared memory of k_cluster_solve (one CTA per SM: all there is)
-static size_t cluster_smem_limit()
-{
-    return 227 * 1024 - 8 * 1024;  // 8 KB for its static shared memory
-}
-
 static void cluster_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute *at, int C, bool resident, int grid,
                            size_t smem, cudaStream_t stream)
 {
@@ -1649,16 +1643,9 @@ static size_t cluster_slice_bytes(const HPRQPMatrixCSR &M, int vw, int C)
     return 16 * (2 * most + ((most + 1) >> 1));
 }
 
-// whether instance k can be solved by a cluster of C CTAs: every CTA has
-// rows (the exchanges of a step order the CTAs through their rows) and the
-// vectors fit
 static bool cluster_fits(const HPRQPBatch *b, size_t k, int C)
 {
-    const long long n = (long long)b->models[k].Q.ncol, m = (long long)b->models[k].A.nrow;
-    const int vw = instance_vw(b, k);
-    if (vw % C != 0 || n < 1 || n > kClMaxLen || m > kClMaxLen) return false;
-    if (C > 1 && (m < 1 || (long long)(C - 1) * (vw / C) * ((n + vw - 1) / vw) >= n)) return false;
-    return cluster_vec_bytes((int)n, (int)m, vw, C) <= cluster_smem_limit();
+    return cluster_fits((long long)b->models[k].Q.ncol, (long long)b->models[k].A.nrow, instance_vw(b, k), C);
 }
 
 static bool cluster_resident(const HPRQPBatch *b, size_t k, int C)
@@ -1667,10 +1654,10 @@ static bool cluster_resident(const HPRQPBatch *b, size_t k, int C)
     const int vw = instance_vw(b, k);
     return cluster_vec_bytes((int)M.Q.ncol, (int)M.A.nrow, vw, C) + cluster_slice_bytes(M.Q, vw, C) +
                cluster_slice_bytes(M.A, vw, C) + cluster_slice_bytes(M.AT, vw, C) + 64 <=
-           cluster_smem_limit();
+           kClSmemLimit;
 }
 
-// clusters of C CTAs the device holds at once (asked once per device)
+// clusters of C CTAs the device, which is current, holds at once (asked until it has answered)
 static int max_clusters(int device, int sms, int C)
 {
     if (C <= 1) return sms;
@@ -1680,7 +1667,7 @@ static int max_clusters(int device, int sms, int C)
     auto it = known.find({device, C});
     if (it != known.end()) return it->second;
     const void *kern = cluster_kernel_of(C, true);
-    const size_t smem = cluster_smem_limit();
+    const size_t smem = kClSmemLimit;
     cudaLaunchConfig_t cfg = {};
     cudaLaunchAttribute at[1];
     cluster_config(cfg, at, C, true, C, smem, nullptr);
@@ -1689,10 +1676,20 @@ static int max_clusters(int device, int sms, int C)
         (C > 8 && cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) ||
         cudaOccupancyMaxActiveClusters(&c, kern, &cfg) != cudaSuccess) {
         cudaGetLastError();
-        c = 0;
+        return 0;
     }
     known[{device, C}] = c;
     return c;
+}
+
+static void cluster_caps(const HPRQPBatch *b, int (&cap)[5])
+{
+    for (int l = 0; l < 5; ++l) cap[l] = max_clusters(b->device, b->num_sms, 1 << l);
+}
+
+static int smallest_cluster(const HPRQPBatch *b, size_t k, const int (&cap)[5])
+{
+    return smallest_cluster((long long)b->models[k].Q.ncol, (long long)b->models[k].A.nrow, instance_vw(b, k), cap);
 }
 
 // Microseconds of one iteration of instance k, measured on the batch recipe
@@ -1724,20 +1721,18 @@ static bool choose_clusters(const std::vector<Item> &items, bool fresh, std::vec
 {
     const size_t N = items.size();
     if (N == 0) return true;
-    const int device = items[0].b->device, sms = items[0].b->num_sms;
+    const int sms = items[0].b->num_sms;
     C.assign(N, 0);
     std::vector<double> t(N);
     std::priority_queue<std::pair<double, size_t>> longest;
     int cap[5];
-    for (int l = 0; l < 5; ++l) cap[l] = max_clusters(device, sms, 1 << l);
+    cluster_caps(items[0].b, cap);
     for (size_t j = 0; j < N; ++j) {
         const HPRQPBatch *b = items[j].b;
         const size_t k = items[j].k;
-        int c = cluster_fits(b, k, 1) ? 1 : 0;
-        if (!c && !fresh) {  // smallest cluster that holds it
-            for (c = 2; c <= 16 && !cluster_fits(b, k, c); c <<= 1) {}
-            if (c > 16) return false;
-        }
+        int c = smallest_cluster(b, k, cap);
+        if (fresh && c > 1) c = 0;
+        if (!fresh && !c) return false;
         t[j] = iteration_us(b, k, c);
         if (fresh && c && iteration_us(b, k, 0) <= t[j]) {
             c = 0;
@@ -1988,9 +1983,6 @@ static HPRQPStatus batch_create_impl(size_t K, const size_t *var_offsets, const 
         I.n = (int)M.Q.ncol;
         I.m = (int)M.A.nrow;
         I.obj_constant = M.obj_constant;
-        I.movable = 0;
-        for (int C = 16; C >= 1; C >>= 1) I.movable |= cluster_fits(b, k, C);
-        b->hold_change += !I.movable;
         // every instance's entries start on a 4-entry (16-byte) boundary, so
         // cta_spmv can read aligned quads of indices and values
         qnz += (M.Q.nnz + 3) & ~size_t(3);
@@ -2084,6 +2076,12 @@ static HPRQPStatus batch_create_impl(size_t K, const size_t *var_offsets, const 
         cudaDeviceGetAttribute(&b->num_sms, cudaDevAttrMultiProcessorCount, device_number) != cudaSuccess ||
         !(b->stream = pool_stream()))
         return fail(HPRQP_STATUS_NOT_IMPLEMENTED);
+    int cap[5];
+    cluster_caps(b, cap);
+    for (size_t k = 0; k < K; ++k) {
+        b->inst[k].movable = smallest_cluster(b, k, cap) > 0;
+        b->hold_change += !b->inst[k].movable;
+    }
     BatchArgs &G = b->args;
     G.K = (int)K;
     int *d_qrp, *d_arp, *d_atrp, *d_qci, *d_aci, *d_atci;
@@ -2223,7 +2221,7 @@ static HPRQPStatus phase_launch(HPRQPBatch *b, SolveLaunch &L, const int *order,
             for (size_t e = g.first; res[s] && e < g.first + g.count; ++e)
                 res[s] = cluster_resident(b, (size_t)b->phase_ids[e], g.C);
             const void *kern = cluster_kernel_of(g.C, res[s]);
-            smem[s] = cluster_smem_limit();
+            smem[s] = kClSmemLimit;
             B_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem[s]));
             if (g.C > 8) B_CK(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
             const int clusters = std::max(1, std::min((int)g.count, max_clusters(b->device, b->num_sms, g.C)));

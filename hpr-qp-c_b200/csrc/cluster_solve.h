@@ -33,6 +33,30 @@ __host__ __device__ __forceinline__ size_t cluster_vec_bytes(int n, int m, int v
     return 8 * (d + 1) + 4 * ((2 * (nl + 1) + ml + 1 + 3) & ~size_t(3));
 }
 
+// dynamic shared memory of k_cluster_solve: one CTA per SM, all there is but
+// 8 KB for its static shared memory
+constexpr size_t kClSmemLimit = 227 * 1024 - 8 * 1024;
+
+// whether an instance whose one-CTA shape has vw warps can be solved by a
+// cluster of C CTAs: every CTA has rows (the exchanges of a step order the
+// CTAs through their rows) and the vectors fit
+inline bool cluster_fits(long long n, long long m, int vw, int C)
+{
+    if (vw % C != 0 || n < 1 || n > kClMaxLen || m > kClMaxLen) return false;
+    if (C > 1 && (m < 1 || (long long)(C - 1) * (vw / C) * ((n + vw - 1) / vw) >= n)) return false;
+    return cluster_vec_bytes((int)n, (int)m, vw, C) <= kClSmemLimit;
+}
+
+// the smallest cluster that can, of the sizes the device holds (a part of a
+// GPU may have no room for large ones; cap[l]: clusters of 2^l CTAs at once);
+// 0: none
+inline int smallest_cluster(long long n, long long m, int vw, const int cap[5])
+{
+    for (int l = 0; l < 5; ++l)
+        if (cap[l] > 0 && cluster_fits(n, m, vw, 1 << l)) return 1 << l;
+    return 0;
+}
+
 // Kernel for clusters of C CTAs; resident: every instance's matrices fit the
 // CTAs' shared memory (no code for streaming them).
 template <int C>
