@@ -48,3 +48,55 @@ def test_movable_instances_do_not_wait_for_others(engine_lib):
     assert r.status[-1] == 5 and 0 < r.iter[-1] < 60000, (r.status[-1], r.iter[-1])
     np.testing.assert_array_equal(r.status[:-1], 4)
     np.testing.assert_array_equal(r.iter[:-1], 60000)
+
+
+def _mixed(kind):
+    """Shapes that a large batch leaves to k_batch_solve: 640-thread ones whose
+    matrices are dense enough, 1024-thread ones, and small ones that the
+    one-CTA form of k_cluster_solve takes."""
+    out = []
+    diag = kind == "diagonal"
+    for i, (n, m, da, dm) in enumerate([(600, 300, 0.07 if diag else 0.03, 0.01),
+                                        (320, 310, 0.13 if diag else 0.07, 0.03),
+                                        (640, 640, 0.03 if diag else 0.012, 0.01), (97, 33, 0.1, 0.1),
+                                        (700, 300, 0.02, 0.01), (1250, 400, 0.01, 0.005)]):
+        inst = instances.plain_qp(300 + i, n=n, m=m, a_density=da, m_rows=n // 3, m_density=dm, n_eq=m // 3)
+        if kind == "free":
+            free = np.random.default_rng(i).random(n) < 0.95
+            inst.l[free], inst.u[free] = -np.inf, np.inf
+        if diag:
+            inst.Q = instances.CSR(n, n, np.arange(n + 1), np.arange(n), np.random.default_rng(i).uniform(0.1, 2.0, n))
+        out.append(inst)
+    return out
+
+
+@pytest.mark.parametrize("count", [200, 312])
+@pytest.mark.parametrize("kind", ["boxed", "free", "diagonal"])
+def test_every_copy_gets_the_same_bits(engine_lib, kind, count):
+    """Copies of six QPs, 353 steps with restarts: most end on the kernel that
+    they started on, the last quarter of the running ones are handed over to
+    clusters, and none of it shows.  With more than two instances per SM each
+    also equals the solve of it alone, on a cluster from the start."""
+    from hprqp.batch import Batch, pack
+
+    insts = _mixed(kind)
+    kw = dict(stoptol=1e-30, max_iter=353)
+    b = Batch(pack([insts[i % 6] for i in range(count)]))
+    b.solve(**kw)
+    r = b.results()
+    parts = {f: b.split(getattr(r, f), "y" if f == "y" else "x") for f in ("x", "y", "z", "w")}
+    scalars = ("objective", "residual", "gap", "sigma", "iter", "status")
+    b.close()
+    for i, inst in enumerate(insts):
+        want = {f: parts[f][i] for f in parts} | {f: getattr(r, f)[i] for f in scalars}
+        if count > 296:
+            alone = Batch(pack([inst]))
+            alone.solve(**kw)
+            s = alone.results()
+            alone.close()
+            want = {f: getattr(s, f) for f in parts} | {f: getattr(s, f)[0] for f in scalars}
+        for k in range(i, count, 6):
+            for f in parts:
+                np.testing.assert_array_equal(parts[f][k], want[f], err_msg=f"{f} of copy {k}")
+            for f in scalars:
+                assert getattr(r, f)[k] == want[f], (f, k)
