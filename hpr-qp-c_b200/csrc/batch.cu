@@ -606,7 +606,7 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
                     const double z_raw = xi + sigma * (-V.Qw[i] + aty - V.c[i]);
                     const double xb = clampd(z_raw, V.l[i], V.u[i]);
                     const double xh = 2.0 * xb - xi;
-                    const double wb = diag ? w_bar_diag(V.fact1[i], wi, V.fact2[i], xh) : f1s * wi + f2s * xh;
+                    const double wb = diag ? w_bar_of(V.fact1[i], wi, V.fact2[i], xh) : w_bar_of(f1s, wi, f2s, xh);
                     if (full) {
                         V.x_bar[i] = xb;
                         V.z_bar[i] = (xb - z_raw) / sigma;
@@ -614,9 +614,9 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
                         V.dw[i] = wb - wi;
                     }
                     V.x_hat[i] = xh;
-                    V.x[i] = h2 * xh + h1 * V.last_x[i];
+                    V.x[i] = average(h2, xh, h1, V.last_x[i]);
                     V.w_bar[i] = wb;
-                    V.w[i] = h2 * (2.0 * wb - wi) + h1 * V.last_w[i];
+                    V.w[i] = average(h2, 2.0 * wb - wi, h1, V.last_w[i]);
                 };
                 if (m > 0) cta_spmv<kBT>(AT, V.y, upd);
                 else
@@ -625,7 +625,7 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
                 cta_spmv<kBT>(Q, V.w_bar, [&](int i, double qwb) {
                     const double qw = V.Qw[i];
                     V.Qw_bar[i] = qwb;
-                    V.Qw[i] = h2 * (2.0 * qwb - qw) + h1 * V.last_Qw[i];
+                    V.Qw[i] = average(h2, 2.0 * qwb - qw, h1, V.last_Qw[i]);
                     V.tempv[i] = V.x_hat[i] + sigma * (qw - qwb);
                 });
                 __syncthreads();
@@ -642,8 +642,8 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
                         V.z_bar[i] = (xb - z_raw) / sigma;
                         V.dx[i] = xb - xi;
                     }
-                    V.x[i] = h2 * xh + h1 * V.last_x[i];
-                    V.w_bar[i] = diag ? w_bar_diag(V.fact1[i], wi, V.fact2[i], xh) : f1s * wi + f2s * xh;
+                    V.x[i] = average(h2, xh, h1, V.last_x[i]);
+                    V.w_bar[i] = diag ? w_bar_of(V.fact1[i], wi, V.fact2[i], xh) : w_bar_of(f1s, wi, f2s, xh);
                 });
                 __syncthreads();
                 if (m > 0) {
@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
                         V.dy[i] = yb - yi;
                         V.s[i] = sp;
                     }
-                    V.y[i] = h2 * (2.0 * yb - yi) + h1 * V.last_y[i];
+                    V.y[i] = average(h2, 2.0 * yb - yi, h1, V.last_y[i]);
                 });
                 __syncthreads();
             }
@@ -681,8 +681,8 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
                         V.w_bar[i] = wbn;
                         V.ATy_bar[i] = atyb;
                     }
-                    V.w[i] = h1 * V.last_w[i] + h2 * (2.0 * wbn - wi);
-                    V.ATy[i] = h1 * V.last_ATy[i] + h2 * (2.0 * atyb - aty);
+                    V.w[i] = average(h2, 2.0 * wbn - wi, h1, V.last_w[i]);
+                    V.ATy[i] = average(h2, 2.0 * atyb - aty, h1, V.last_ATy[i]);
                 };
                 if (m > 0) cta_spmv<kBT>(AT, V.y_bar, w2);
                 else
@@ -724,25 +724,7 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
             cta_allreduce<4, kBW>(a, ops4, s_red, s_out);
             cta_allreduce<2, kBW>(b, ops2, s_red, s_out);
             cta_allreduce<3, kBW>(c3, ops3, s_red, s_out);
-            const double sigma = S.sigma, lA = S.lA, lQ = S.lQ;
-            double m1 = 0.0, m3 = 0.0, m2 = (1.0 / sigma) * a[0];
-            m2 -= 2.0 * a[1];
-            if (m > 0) {
-                m1 = sigma * lA * b[1];
-                m1 -= 2.0 * sigma * c3[0];
-                m2 += 2.0 * b[0];
-                if (S.q_is_diag) {
-                    m3 = c3[2];
-                    m1 += sigma * a[2];
-                } else {
-                    m3 = (sigma * sigma) / (1.0 + sigma * lQ) * c3[1];
-                    m1 += sigma * lQ * a[3];
-                }
-            } else if (!S.q_is_diag) {
-                m1 = sigma * lQ * a[3];
-            }
-            m2 += m1 > 0.0 ? m1 : 0.0;
-            return sqrt((m2 > 0.0 ? m2 : 0.0) + (m3 > 0.0 ? m3 : 0.0));
+            return m_norm_of(S.sigma, S.lA, S.lQ, m > 0, S.q_is_diag, a, b, c3);
         };
 
         // ---- sigma update (reference control.cu:334-529) ----------------------
@@ -780,19 +762,8 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
             cta_allreduce<2, kBW>(d, ops2, s_red, s_out);
             cta_allreduce<3, kBW>(e3, ops3, s_red, s_out);
             cta_allreduce<1, kBW>(f1v, ops1, s_red, s_out);
-            double a = 0.0, b = d[0], c_term = 0.0, d_term = 0.0;
-            if (m > 0) a = lA * d[1] - 2.0 * e3[0];
-            if (S.q_is_diag) {
-                a += e3[1];
-            } else {
-                a += lQ * e3[2];
-                if (m > 0) {
-                    c_term = f1v[0];
-                    d_term = lQ;
-                }
-            }
-            a = fmax(a, 1e-12);
-            b = fmax(b, 1e-12);
+            const double a = sigma_slope(lA, lQ, m > 0, S.q_is_diag, d[1], e3[0], e3[1], e3[2]), b = fmax(d[0], 1e-12);
+            const double c_term = m > 0 ? f1v[0] : 0.0, d_term = m > 0 ? lQ : 0.0;
             double est;
             if (S.q_is_diag && m > 0) {
                 // golden section with a CTA-wide sum per probe
@@ -854,8 +825,8 @@ __global__ void __launch_bounds__(BT, ctas_per_sm(BT)) k_batch_solve(const Batch
                 est = clampd(est, 1e-12, 1e12);
                 const double fact =
                     (S.best_gap > 0.0 && isfinite(S.best_gap)) ? exp(-0.05 * (S.current_gap / S.best_gap)) : 1.0;
-                const double cand =
-                    exp(fact * log(est) + (1.0 - fact) * log(S.best_sigma > 0.0 ? S.best_sigma : sigma_old));
+                const double best = log(S.best_sigma > 0.0 ? S.best_sigma : sigma_old);
+                const double cand = exp(two_products(1.0 - fact, best, fact, log(est)));
                 double kappa = 1.0;
                 const double t1 = fmax(fmin(S.rd, S.rp), fmin(S.gap, S.current_gap));
                 if (t1 <= 9e-10 && S.rp > 0.0) {

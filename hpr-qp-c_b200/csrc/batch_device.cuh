@@ -125,19 +125,61 @@ __device__ __forceinline__ double clampd(double v, double lo, double hi)
     return v < lo ? lo : (v > hi ? hi : v);
 }
 
-// The factors of a diagonal Q and w_bar, rounded one way wherever they are
-// compiled: an instance may start in k_batch_solve and go on in
+// What both batch kernels compute from two products, rounded one way wherever
+// it is compiled: an instance may start in k_batch_solve and go on in
 // k_cluster_solve, at a moment that depends on the others, and must not show
-// where it did.  (Left to the compiler, sigma d is fused into 1 + sigma d in
-// one kernel and shared with fact1 in the other.)
+// where it did.  (Left to the compiler, either product of a sum of two may be
+// the fused one, and a product that is needed twice is not fused at all: sigma
+// d was fused into 1 + sigma d in one kernel and shared with fact1 in the
+// other.)
+// p a + q b, the first product fused
+__device__ __forceinline__ double two_products(double p, double a, double q, double b)
+{
+    return fma(p, a, __dmul_rn(q, b));
+}
+// the Halpern average h2 now + h1 anchor
+__device__ __forceinline__ double average(double h2, double now, double h1, double anchor)
+{
+    return two_products(h2, now, h1, anchor);
+}
 __device__ __forceinline__ double diag_inverse(double sigma, double d) { return 1.0 / fma(sigma, d, 1.0); }
 __device__ __forceinline__ double diag_fact1(double sigma, double d, double inv)
 {
     return __dmul_rn(__dmul_rn(sigma, d), inv);
 }
-__device__ __forceinline__ double w_bar_diag(double f1, double w, double f2, double x_hat)
+__device__ __forceinline__ double w_bar_of(double f1, double w, double f2, double x_hat)
 {
-    return fma(f1, w, __dmul_rn(f2, x_hat));
+    return two_products(f1, w, f2, x_hat);
+}
+// M-norm from its sums (reference control.cu:243-332); a: dx dx, dx Qdw,
+// Qdw Qdw, dw Qdw; b: A'dy dx, dy dy; c: Qdw A'dy, A'dy QA'dy, A'dy M QA'dy
+__device__ __forceinline__ double m_norm_of(double sigma, double lA, double lQ, bool rows, bool diag, const double *a,
+                                            const double *b, const double *c)
+{
+    double m1 = 0.0, m3 = 0.0, m2 = two_products(1.0 / sigma, a[0], -2.0, a[1]);
+    if (rows) {
+        m1 = two_products(__dmul_rn(sigma, lA), b[1], -2.0 * sigma, c[0]);
+        m2 += 2.0 * b[0];
+        if (diag) {
+            m3 = c[2];
+            m1 = fma(sigma, a[2], m1);
+        } else {
+            m3 = (sigma * sigma) / fma(sigma, lQ, 1.0) * c[1];
+            m1 = fma(__dmul_rn(sigma, lQ), a[3], m1);
+        }
+    } else if (!diag) {
+        m1 = sigma * lQ * a[3];
+    }
+    m2 += m1 > 0.0 ? m1 : 0.0;
+    return sqrt((m2 > 0.0 ? m2 : 0.0) + (m3 > 0.0 ? m3 : 0.0));
+}
+// the coefficient of sigma in the sigma estimate (reference control.cu:334-529)
+__device__ __forceinline__ double sigma_slope(double lA, double lQ, bool rows, bool diag, double dy_dy, double dqw_atdy,
+                                              double dqw_dqw, double dw_dqw)
+{
+    double a = rows ? two_products(lA, dy_dy, -2.0, dqw_atdy) : 0.0;
+    a += diag ? dqw_dqw : __dmul_rn(lQ, dw_dqw);
+    return fmax(a, 1e-12);
 }
 
 // CTA-shared control state of the instance being solved

@@ -925,8 +925,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
         auto step = [&](bool full, int mail, long long next_iter, double h1) {
             const double sigma = S.sigma, h2 = 1.0 - h1;
             const double f2s = s_k[0], f1s = s_k[1];
-            // (the rounding k_batch_solve's code has)
-            auto average = [&](double now, double anchor) { return fma(h2, now, __dmul_rn(h1, anchor)); };
+            auto average = [&](double now, double anchor) { return hpr::average(h2, now, h1, anchor); };
             if (noC) {
                 auto upd = [&](int i, double aty) {
                     const int gi = nr0 + i;
@@ -935,7 +934,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
                     const double z_raw = xi + sigma * (-own[kClNOwn * i + kQw] + aty - own[kClNOwn * i + kC]);
                     const double xb = clampd(z_raw, own[kClNOwn * i + kL], own[kClNOwn * i + kU]);
                     const double xh = 2.0 * xb - xi;
-                    const double wb = diag ? w_bar_diag(V.fact1[nr0 + i], wi, V.fact2[nr0 + i], xh) : f1s * wi + f2s * xh;
+                    const double wb = w_bar_of(diag ? V.fact1[nr0 + i] : f1s, wi, diag ? V.fact2[nr0 + i] : f2s, xh);
                     push(G2 + gi, wb, kBarWb);
                     if (full) {
                         V.x_bar[gi] = xb;
@@ -965,7 +964,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
                     const double z_raw = xi + sigma * (-qw + own[kClNOwn * i + kAty] - own[kClNOwn * i + kC]);
                     const double xb = clampd(z_raw, own[kClNOwn * i + kL], own[kClNOwn * i + kU]);
                     const double xh = 2.0 * xb - xi;
-                    const double wb = diag ? w_bar_diag(V.fact1[nr0 + i], wi, V.fact2[nr0 + i], xh) : f1s * wi + f2s * xh;
+                    const double wb = w_bar_of(diag ? V.fact1[nr0 + i] : f1s, wi, diag ? V.fact2[nr0 + i] : f2s, xh);
                     push(G2 + gi, wb, kBarWb);
                     own[kClNOwn * i + kQw] = qw;
                     own[kClNOwn * i + kXh] = xh;
@@ -1056,25 +1055,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
             }
             finish(m > 0 ? 9 : 4, 0u);
             const double *a = s_out, *b = s_out + 4, *c3 = s_out + 6;
-            const double sigma = S.sigma, lA = S.lA, lQ = S.lQ;
-            double m1 = 0.0, m3 = 0.0, m2 = (1.0 / sigma) * a[0];
-            m2 -= 2.0 * a[1];
-            if (m > 0) {
-                m1 = sigma * lA * b[1];
-                m1 -= 2.0 * sigma * c3[0];
-                m2 += 2.0 * b[0];
-                if (diag) {
-                    m3 = c3[2];
-                    m1 += sigma * a[2];
-                } else {
-                    m3 = (sigma * sigma) / (1.0 + sigma * lQ) * c3[1];
-                    m1 += sigma * lQ * a[3];
-                }
-            } else if (!diag) {
-                m1 = sigma * lQ * a[3];
-            }
-            m2 += m1 > 0.0 ? m1 : 0.0;
-            return sqrt((m2 > 0.0 ? m2 : 0.0) + (m3 > 0.0 ? m3 : 0.0));
+            return m_norm_of(S.sigma, S.lA, S.lQ, m > 0, diag, a, b, c3);
         };
 
         // ---- sigma update (reference control.cu:334-529) ----------------------
@@ -1108,19 +1089,8 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
             fold_rows(m > 0 ? n : 0, per_n, 5, 1, 0u, [&](int i, double *e) { e[0] += V.ATdy[i] * V.QATdy[i]; });
             finish(6, 0u);
             const double e_dx = s_out[0], e_dy = s_out[1], e0 = s_out[2], e1 = s_out[3], e2 = s_out[4], e_f = s_out[5];
-            double a = 0.0, b = e_dx, c_term = 0.0, d_term = 0.0;
-            if (m > 0) a = lA * e_dy - 2.0 * e0;
-            if (diag) {
-                a += e1;
-            } else {
-                a += lQ * e2;
-                if (m > 0) {
-                    c_term = e_f;
-                    d_term = lQ;
-                }
-            }
-            a = fmax(a, 1e-12);
-            b = fmax(b, 1e-12);
+            const double a = sigma_slope(lA, lQ, m > 0, diag, e_dy, e0, e1, e2), b = fmax(e_dx, 1e-12);
+            const double c_term = m > 0 ? e_f : 0.0, d_term = m > 0 ? lQ : 0.0;
             double est = 0.0;
             if (diag && m > 0) {
                 // golden section with a cluster-wide sum per probe
@@ -1185,8 +1155,8 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
                 est = clampd(est, 1e-12, 1e12);
                 const double fact =
                     (S.best_gap > 0.0 && isfinite(S.best_gap)) ? exp(-0.05 * (S.current_gap / S.best_gap)) : 1.0;
-                const double cand =
-                    exp(fact * log(est) + (1.0 - fact) * log(S.best_sigma > 0.0 ? S.best_sigma : sigma_old));
+                const double best = log(S.best_sigma > 0.0 ? S.best_sigma : sigma_old);
+                const double cand = exp(two_products(1.0 - fact, best, fact, log(est)));
                 double kappa = 1.0;
                 const double t1 = fmax(fmin(S.rd, S.rp), fmin(S.gap, S.current_gap));
                 if (t1 <= 9e-10 && S.rp > 0.0) {
