@@ -221,7 +221,7 @@ static __device__ __forceinline__ bool yield_now(const BatchArgs &B, const BInst
            *(volatile unsigned long long *)B.hold == 0;
 }
 
-// instance I has ended
+// instance I of k_batch_solve has ended (those of k_cluster_solve are movable)
 static __device__ __forceinline__ void count_finished(const BatchArgs &B, const BInst &I)
 {
     atomicAdd(B.finished, 1ull);

@@ -263,7 +263,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
                     B.restarts[k] = 0;
                     B.sigma_out[k] = 0.0;
                     B.seconds_out[k] = 0.0;
-                    count_finished(B, I);
+                    atomicAdd(B.finished, 1ull);  // (no instance here holds a hand-over up)
                 }
             }
             continue;
@@ -934,7 +934,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
                     const double z_raw = xi + sigma * (-own[kClNOwn * i + kQw] + aty - own[kClNOwn * i + kC]);
                     const double xb = clampd(z_raw, own[kClNOwn * i + kL], own[kClNOwn * i + kU]);
                     const double xh = 2.0 * xb - xi;
-                    const double wb = w_bar_of(diag ? V.fact1[nr0 + i] : f1s, wi, diag ? V.fact2[nr0 + i] : f2s, xh);
+                    const double wb = diag ? w_bar_of(V.fact1[nr0 + i], wi, V.fact2[nr0 + i], xh) : w_bar_of(f1s, wi, f2s, xh);
                     push(G2 + gi, wb, kBarWb);
                     if (full) {
                         V.x_bar[gi] = xb;
@@ -964,7 +964,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
                     const double z_raw = xi + sigma * (-qw + own[kClNOwn * i + kAty] - own[kClNOwn * i + kC]);
                     const double xb = clampd(z_raw, own[kClNOwn * i + kL], own[kClNOwn * i + kU]);
                     const double xh = 2.0 * xb - xi;
-                    const double wb = w_bar_of(diag ? V.fact1[nr0 + i] : f1s, wi, diag ? V.fact2[nr0 + i] : f2s, xh);
+                    const double wb = diag ? w_bar_of(V.fact1[nr0 + i], wi, V.fact2[nr0 + i], xh) : w_bar_of(f1s, wi, f2s, xh);
                     push(G2 + gi, wb, kBarWb);
                     own[kClNOwn * i + kQw] = qw;
                     own[kClNOwn * i + kXh] = xh;
@@ -1433,7 +1433,7 @@ __global__ void __launch_bounds__(NT, 1) k_cluster_solve(const ClusterArgs P)
             B.sigma_out[k] = S.sigma;
             B.seconds_out[k] = 1e-9 * (double)(globaltimer_ns() - inst_t0);
             if (B.loop_seconds_out) B.loop_seconds_out[k] = 1e-9 * (double)(globaltimer_ns() - loop_t0);
-            count_finished(B, I);
+            atomicAdd(B.finished, 1ull);
         }
         sync();
         if (MULTI && s_dead) break;
