@@ -41,14 +41,14 @@ ROOT = Path(__file__).resolve().parent
 sys.path.insert(0, str(ROOT / "hpr-qp-c_b200" / "python"))
 sys.path.insert(0, str(ROOT / "oracle"))
 
-# DRAM bytes moved per algorithmic byte by k_batch_solve: ncu on a 300-QP
-# solve of this workload, every instance in k_batch_solve (a 640-thread launch
-# for its 85 instances of n, m <= 640, a 1024-thread launch for the rest, one
-# instance per SM at a time, no shared-memory pool) read+wrote 0.009 +
-# 394.424 GB (dram__bytes_read.sum + dram__bytes_write.sum of both launches)
-# for 512.257 GB of algorithmic bytes; traffic grows with instance-iterations,
-# so the bench scales this ratio by its own solve's algorithmic bytes.
-BATCH_DRAM_PER_ALGO_BYTE = 394.433e9 / 512.257e9
+# DRAM bytes moved per algorithmic byte by a solve: ncu on a 300-QP solve of
+# this workload (68 small instances in k_cluster_solve's one-CTA form, 17 in a
+# 640-thread and 215 in a 1024-thread launch of k_batch_solve, the last ones
+# handed over to clusters) read+wrote 391.10 GB (dram__bytes_read.sum +
+# dram__bytes_write.sum of its seven launches) for 512.257 GB of algorithmic
+# bytes; traffic grows with instance-iterations, so the bench scales this
+# ratio by its own solve's algorithmic bytes.
+BATCH_DRAM_PER_ALGO_BYTE = 391.10e9 / 512.257e9
 METRIC = "solves/s to 1e-6 rel-KKT, batched vs plain on 1 B200; SpMV GB/s vs HBM peak"
 STOPTOL = 1e-6
 BATCH = 4096
@@ -730,10 +730,8 @@ def main():
                     "optimal": e2e_ok},
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": algo_bytes * BATCH_DRAM_PER_ALGO_BYTE,
-                         "traffic_source": "estimate: ncu DRAM bytes of a 300-QP solve of this workload with every "
-                                           "instance in k_batch_solve (the small ones now run in "
-                                           "k_cluster_solve's one-CTA form), scaled by algorithmic bytes "
-                                           "(instance-iterations)",
+                         "traffic_source": "estimate: ncu DRAM bytes of all launches of a 300-QP solve of this "
+                                           "workload, scaled by algorithmic bytes (instance-iterations)",
                          "kernel": "k_batch_solve and k_cluster_solve (one solve: a one-CTA launch for "
                                    "the instances of n, m <= 640 and a 1024-thread launch for the "
                                    "rest, concurrent, the last ones handed to clusters; achieved over "

@@ -72,7 +72,7 @@ constexpr int ctas_per_sm(int bt) { return bt >= 1024 ? 1 : 1024 / bt; }
 // vector loop one entry per thread) and work (nnz(Q) + 2 nnz(A) + n of the
 // preprocessed model) at most kMidCtaMaxWork is solved by a 640-thread CTA
 // (96 registers against 64, one CTA per SM either way), in a launch of its
-// own started first (batch_launch).  Per-iteration times on the 4096-QP
+// own started first (first_phase).  Per-iteration times on the 4096-QP
 // batch recipe: 640 threads 18-24 % faster for n < 640, even or slower
 // above (each vector loop takes two passes), 7-15 % slower for work above
 // 40,000; 768 and 512 threads gave smaller and larger versions of the same
@@ -2814,11 +2814,12 @@ namespace hpr {
 // would end the call late).  The rest is built and uploaded meanwhile and
 // launched on its own stream (its CTAs take the SMs as the first launch's
 // CTAs finish); each part's results are scattered back to the caller's
-// packing.  Each instance is solved by one CTA of the shape a single launch
+// packing.  Each instance sums in the order of the shape a single launch
 // would give it (batches this large take 1024-thread CTAs, and 640-thread
 // CTAs for the instances mid_cta_instance picks, a rule on the instance
-// alone), so the results equal a single launch's bit for bit; each launch
-// keeps its own time limit.
+// alone), so the results equal a single launch's bit for bit; each part keeps
+// its own time limit.  The last running instances of both parts are handed
+// over together, once the second part is launched (BatchArgs::hold).
 constexpr size_t kSplitMinInstances = 1024;
 constexpr double kFirstPartWork = 0.15;
 
@@ -2975,7 +2976,7 @@ HPRQPStatus hprqp_solve_batch(size_t K, const size_t *var_offsets, const size_t 
 namespace hpr {
 
 // Models whose products per iteration stay below this many nonzeros
-// (2 nnz(Q) + 2 nnz(A)) run in one CTA of the batch kernel: a host-driven
+// (2 nnz(Q) + 2 nnz(A)) run as a batch of one: a host-driven
 // iteration costs four kernel launches and the device-wide passes of the
 // plain engine, which small problems cannot fill.  Process-wide; set by
 // hprqp_b200_set_single_cta_max_work.

@@ -63,8 +63,8 @@ HPRQPStatus engine_adjoint(Engine *e, const double *gx, const double *gy, double
 HPRQPStatus solve_gpu_keep(const HPRQPModel *model, const HPRQPParams *params, HPRQPResults *results,
                            Engine **keep);
 
-// Small single QPs: the whole solve in one CTA of the batch kernel (one
-// launch, no host round trips per iteration).  single_cta_eligible() says
+// Small single QPs: the whole solve as a batch of one (one launch, no host
+// round trips per iteration).  single_cta_eligible() says
 // whether solve_gpu takes this path for a model and parameters; the solve
 // fills results like the host loop (iterations, milestones, loop time,
 // objective, residuals, x, y, z, w) and, when log is given, appends one

@@ -258,8 +258,8 @@ HPRQPStatus hpr::solve_gpu_keep(const HPRQPModel *model, const HPRQPParams *para
         print_params_info(params);
     }
     if (!keep && hpr::single_cta_eligible(model, params)) {
-        // the whole solve in one CTA of the batch kernel; the log comes back
-        // with the results and is printed like the host loop prints it
+        // the whole solve as a batch of one; the log comes back with the
+        // results and is printed like the host loop prints it
         std::vector<double> log;
         if (params->verbose) log.resize(hpr::kSingleCtaLogCap * 8);
         size_t nlog = 0;

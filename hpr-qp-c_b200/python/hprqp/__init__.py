@@ -191,8 +191,8 @@ def launch_count() -> int:
 
 def set_single_cta_max_work(max_work: int) -> int:
     """Route solve_gpu: models without cones whose products per iteration
-    touch at most ``max_work`` nonzeros (2 nnz(Q) + 2 nnz(A)) are solved in
-    one CTA of the batch kernel; 0 sends every model through the host-driven
+    touch at most ``max_work`` nonzeros (2 nnz(Q) + 2 nnz(A)) are solved as a
+    batch of one on the device; 0 sends every model through the host-driven
     loop.  Returns the previous value (hprqp_b200_set_single_cta_max_work)."""
     return int(_lib().hprqp_b200_set_single_cta_max_work(int(max_work)))
 

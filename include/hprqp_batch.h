@@ -50,10 +50,14 @@ HPRQPStatus hprqp_batch_create(size_t num_instances, const size_t *var_offsets, 
  * one instance per CTA, taken from a work queue with two ends (half the CTAs
  * take the largest instance left, half the smallest).  In a batch of more
  * than two instances per SM, the instances of at most 640 variables and 640
- * rows with few nonzeros run in a launch of 640-thread CTAs started first,
- * the others in a launch of 1024-thread CTAs beside it; the shape is fixed
- * per instance, so an instance's result does not depend on the rest of the
- * batch or on timing.  Returns when the solve has ended.  May be called
+ * rows with few nonzeros run in launches of their own started first, the
+ * others in a launch of 1024-thread CTAs beside them.  A batch of at most one
+ * instance per SM, and the last running instances of a larger one, run on
+ * thread-block clusters; an instance that no cluster takes (more than 8190
+ * variables or rows, or vectors beyond a cluster's shared memory) stays on
+ * its CTA, and the others are not moved before it has ended.  The order of an
+ * instance's sums is fixed by its size and the batch's, so its result depends
+ * on neither the kernel it runs on nor on timing.  Returns when the solve has ended.  May be called
  * repeatedly; every call starts from the original data, at zero or at the
  * point set by hprqp_batch_set_warm_start. */
 HPRQPStatus hprqp_batch_solve(HPRQPBatch *batch, const HPRQPBatchParams *params);
@@ -91,7 +95,7 @@ HPRQPStatus hprqp_batch_request_abort(HPRQPBatch *batch);
 /* sigma of each instance at the end of the last hprqp_batch_solve. */
 HPRQPStatus hprqp_batch_get_sigma(const HPRQPBatch *batch, double *sigma);
 
-/* Seconds each instance of the last hprqp_batch_solve took on its CTA, from
+/* Seconds each instance of the last hprqp_batch_solve took, from
  * loading its data to writing its results (device clock; instances run
  * concurrently, so these do not add up to the launch time).  The per-solve
  * time a dataset table reports for a batched run. */
